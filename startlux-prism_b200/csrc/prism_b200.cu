@@ -18,8 +18,8 @@
 #include "w8a8_groups.cuh"
 #include "w8a8_g32.cuh"
 #include "w4a8_gemm.cuh"
-#include "w4a8_few.cuh"
 #include "w4a8_gemv.cuh"
+#include "w4a8_mma.cuh"
 #include "w8a8_gemv.cuh"
 #include "mxfp4_gemm.cuh"
 #include "mxfp4_gemv.cuh"
@@ -349,16 +349,6 @@ bool w4a8_tile_only() {
     return v == 1;
 }
 
-// PRISM_B200_W4A8_STAGED=1: the few-rows Q4_K kernel that stages the expanded operand in shared memory (comparison runs).
-bool w4a8_few_staged() {
-    static int v = -1;
-    if (v < 0) {
-        const char* e = getenv("PRISM_B200_W4A8_STAGED");
-        v = (e && e[0] == '1') ? 1 : 0;
-    }
-    return v == 1;
-}
-
 template <int EPI>
 int launch_pair(const int8_t* a, const float* a_s, const int8_t* w, const float* w_s, void* out, long ldo,
                 const int* n_rows, int M, int N, int K, cudaStream_t st) {
@@ -551,85 +541,68 @@ int launch_w4a8(const int8_t* xq, const float* a, const int8_t* xs, int Ma, cons
     if ((rc = tensor_map(&m.d, wd, N, NSB, (uint64_t)N * 4, 64, 1, 1))) return rc;
     auto kern = w4a8::w4a8_kernel<KIND>;
     if ((rc = set_smem(kern, C::SMEM))) return rc;
-    w4a8::Args p{a, out, ldo, n_rows, M, N, K, Ma, epi, nullptr, nullptr, nullptr, nullptr, 1, K / 256, nullptr, nullptr};
+    w4a8::Args p{a, out, ldo, n_rows, M, N, K, Ma, epi};
     const int grid = ((M + 127) / 128) * ((N + 63) / 64);
     kern<<<grid, w4a8::THREADS, C::SMEM, st>>>(m, p);
     PB_CUDA(cudaGetLastError());
     return PB_OK;
 }
 
-// Few activation rows (w4a8_few.cuh): weight tiles of 128 (Q4_K) or 64 (Q6_K) rows against 16 activation rows.
-template <int KIND>
-int launch_w4a8_few(const int8_t* xq, const float* a, const int8_t* xs, int Ma, const void* wq, const void* wsc,
-                    const void* wmn, const float* wd, const float* wdm, void* out, long ldo, const int* n_rows, int M,
-                    int N, int K, int epi, cudaStream_t st, int split = 1, float* ws = nullptr, int* counters = nullptr) {
-    using C = w4a8::FewCfg<KIND>;
-    w4a8::FewMaps m;
+// A decode batch (w4a8_mma.cuh).  Per configuration: 8 * MT activation rows, 16 * NT * WN weight rows and WK super-blocks a
+// round per CTA, ST rounds in flight.
+template <int KIND, int MT, int NT, int WN, int WK, int ST>
+int launch_w4a8_mma(const w4a8::GemvArgs& p, cudaStream_t st) {
+    using C = w4a8::MmaCfg<KIND, MT, NT, WN, WK, ST>;
+    static_assert(C::SMEM <= 232448, "shared memory of a CTA");
+    auto kern = w4a8::w4a8_mma_kernel<KIND, MT, NT, WN, WK, ST>;
     int rc;
-    const uint64_t NSB = K / 256;
-    if ((rc = tensor_map(&m.x, xq, K, M, K, 128, w4a8::FEW_NB, 0))) return rc;
-    if (KIND == w4a8::KIND_Q4K) {
-        if ((rc = tensor_map(&m.wq, wq, K / 2, N, K / 2, 128, 128, 0))) return rc;
-        if ((rc = tensor_map(&m.xs, xs, (uint64_t)Ma * 4, NSB, (uint64_t)Ma * 16, w4a8::FEW_NB * 4, 1, 3))) return rc;
-        if ((rc = tensor_map(&m.sc, wsc, (uint64_t)N * 2, NSB, (uint64_t)N * 8, 256, 1, 3))) return rc;
-        if ((rc = tensor_map(&m.mn, wmn, (uint64_t)N * 2, NSB, (uint64_t)N * 8, 256, 1, 3))) return rc;
-        if ((rc = tensor_map(&m.dm, wdm, N, NSB, (uint64_t)N * 4, 128, 1, 1))) return rc;
-    } else {
-        if ((rc = tensor_map(&m.wq, wq, K, N, K, 128, 64, 0))) return rc;
-        if ((rc = tensor_map(&m.sc, wsc, (uint64_t)N * 4, NSB, (uint64_t)N * 16, 256, 1, 3))) return rc;
-        m.xs = m.x;
-        m.mn = m.x;
-        m.dm = m.x;
-    }
-    if ((rc = tensor_map(&m.d, wd, N, NSB, (uint64_t)N * 4, C::TILE_N, 1, 1))) return rc;
-    const int nsb = K / 256;
-    if (split > nsb) split = nsb;
-    const int sps = (nsb + split - 1) / split;
-    split = (nsb + sps - 1) / sps;                                    // no empty slice
-    w4a8::Args p{a, out, ldo, n_rows, M, N, K, Ma, epi, (const uint8_t*)wsc, (const uint8_t*)wmn, wd, wdm, split, sps, ws,
-                 counters};
-    // the row tiles of one weight tile are neighbours in launch order: the weights of all but the first come from L2
-    dim3 grid((M + w4a8::FEW_NB - 1) / w4a8::FEW_NB, (N + C::TILE_N - 1) / C::TILE_N);
-    if (KIND == w4a8::KIND_Q4K && !w4a8_few_staged()) {
-        // Q4_K: the expanded operand goes through tensor memory
-        if ((rc = set_smem(w4a8::w4a8_few_q4k_tm_kernel<false>, w4a8::TmCfg::SMEM))) return rc;
-        if ((rc = set_smem(w4a8::w4a8_few_q4k_tm_kernel<true>, w4a8::TmCfg::SMEM))) return rc;
-        grid.z = split;
-        if (split > 1) w4a8::w4a8_few_q4k_tm_kernel<true><<<grid, w4a8::FEW_THREADS, w4a8::TmCfg::SMEM, st>>>(m, p);
-        else w4a8::w4a8_few_q4k_tm_kernel<false><<<grid, w4a8::FEW_THREADS, w4a8::TmCfg::SMEM, st>>>(m, p);
-        PB_CUDA(cudaGetLastError());
-        return PB_OK;
-    }
-    auto kern = w4a8::w4a8_few_kernel<KIND>;
     if ((rc = set_smem(kern, C::SMEM))) return rc;
-    if (KIND == w4a8::KIND_Q6K) grid.z = split;
-    else p.split = 1;
-    kern<<<grid, w4a8::FEW_THREADS, C::SMEM, st>>>(m, p);
+    const unsigned grid = (unsigned)((p.N + C::ROWS - 1) / C::ROWS) * (unsigned)((p.M + C::MP - 1) / C::MP);
+    kern<<<grid, C::THREADS, C::SMEM, st>>>(p);
     PB_CUDA(cudaGetLastError());
     return PB_OK;
 }
 
-// One to four activation rows: integer dot products on the CUDA cores (w4a8_gemv.cuh).
+// Which one: measured on 5120 / 6144 / 34816 x 5120 (Q4_K) and 1024 x 5120, 5120 x 17408 (Q6_K), one launch, weights from HBM.
+// With N / 16 warps already eight per SM (`wide`) every warp walks through the whole of K; below that K is split over
+// the CTA's warps and a CTA takes 16 weight rows, so that 5120 rows still are two CTAs per SM (Q4_K, 8 rows: wide
+// 21.4 us whole against 26.8 split on 34816 rows, 10.3 against 7.0 on 5120).  More rows than 16 take their activation rows in blocks of 16
+// there (14.9 us against 15.8 at 32 rows in one block).
+template <int KIND>
+int launch_w4a8_few(const w4a8::GemvArgs& p, cudaStream_t st) {
+    if (KIND == w4a8::KIND_Q4K) {
+        const bool wide = p.N >= 16 * 8 * sm_count();
+        if (p.M <= 8) return wide ? launch_w4a8_mma<KIND, 1, 1, 4, 1, 4>(p, st) : launch_w4a8_mma<KIND, 1, 1, 1, 4, 3>(p, st);
+        if (!wide) return launch_w4a8_mma<KIND, 2, 1, 1, 4, 2>(p, st);
+        return p.M <= 16 ? launch_w4a8_mma<KIND, 2, 2, 4, 1, 3>(p, st) : launch_w4a8_mma<KIND, 4, 1, 4, 2, 2>(p, st);
+    }
+    if (p.N <= 16 * sm_count())
+        return p.M <= 16 ? launch_w4a8_mma<KIND, 1, 1, 1, 4, 4>(p, st) : launch_w4a8_mma<KIND, 2, 1, 1, 4, 3>(p, st);
+    if (p.M <= 8) return launch_w4a8_mma<KIND, 1, 1, 2, 4, 2>(p, st);
+    return p.M <= 16 ? launch_w4a8_mma<KIND, 2, 2, 2, 4, 2>(p, st) : launch_w4a8_mma<KIND, 4, 1, 4, 2, 2>(p, st);
+}
+
+// One or two activation rows against Q6_K: integer dot products on the CUDA cores (w4a8_gemv.cuh).
 template <int MR>
-int launch_w4a8_gemv(int kind, const w4a8::GemvArgs& p, cudaStream_t st) {
+int launch_w4a8_gemv(const w4a8::GemvArgs& p, cudaStream_t st) {
     constexpr int R = w4a8::GEMV_R;
     const int grid = (p.N + 4 * R - 1) / (4 * R);                  // eight weight rows per CTA
-    auto split_k = kind == 0 ? w4a8::w4a8_gemv_q4k_kernel<MR, R, true> : w4a8::w4a8_gemv_q6k_kernel<MR, R, true>;
-    auto whole_k = kind == 0 ? w4a8::w4a8_gemv_q4k_kernel<MR, R, false> : w4a8::w4a8_gemv_q6k_kernel<MR, R, false>;
+    auto split_k = w4a8::w4a8_gemv_q6k_kernel<MR, R, true>;
+    auto whole_k = w4a8::w4a8_gemv_q6k_kernel<MR, R, false>;
     // few rows: two to four warps per CTA share the rows' super-blocks (exact: the chain runs in order afterwards);
     // the most warps with which the whole grid is resident at once (a second, short wave would double the time)
     const size_t smem = (size_t)(p.K >> 8) * 4 * R * MR * sizeof(float);
     if (grid < 8 * sm_count() && smem <= 48 * 1024) {
-        static int resident_dev[kMaxDevices][2][5] = {};           // [device][kind][warps] CTAs per SM, 0 = not asked yet
-        int (&resident)[2][5] = resident_dev[current_device()];
+        static int resident_dev[kMaxDevices][5] = {};              // [device][warps] CTAs per SM, 0 = not asked yet
+        int (&resident)[5] = resident_dev[current_device()];
         int kw = 2;
         for (int k = 4; k >= 2; --k) {
-            if (!resident[kind][k]) {
+            if (!resident[k]) {
                 int nb = 0;
                 PB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, split_k, 32 * k, 16 * 1024));
-                resident[kind][k] = nb > 0 ? nb : 1;
+                resident[k] = nb > 0 ? nb : 1;
             }
-            if ((long)grid <= (long)resident[kind][k] * sm_count()) {
+            if ((long)grid <= (long)resident[k] * sm_count()) {
                 kw = k;
                 break;
             }
@@ -706,7 +679,7 @@ bool w8a8_no_gemv() {
     return v == 1;
 }
 
-// PRISM_B200_W4A8_NO_GEMV=1 keeps the tensor-core kernels for one to four rows (comparison runs).
+// PRISM_B200_W4A8_NO_GEMV=1 keeps the tensor-core kernels for one and two Q6_K rows (comparison runs).
 bool w4a8_no_gemv() {
     static int v = -1;
     if (v < 0) {
@@ -1444,36 +1417,21 @@ int pb_w4a8_gemm(const int8_t* xq, const float* a, const int8_t* xs, int Ma, int
     if (K % 256 || N % 4 || ldo < N) return PB_UNSUPPORTED_SHAPE;
     if (!aligned16(xq) || !aligned16(wq) || !aligned16(wsc) || !aligned16(wd) || (kind == 0 && (!aligned16(xs) ||
         !aligned16(wmn) || !aligned16(wdm)))) return PB_BAD_ARGUMENT;
-    // one or two rows, or up to eight against a matrix of few rows: the CUDA-core kernel (measured: from three rows on
-    // a 34816-row matrix the tensor-core kernel below is level or ahead)
-    if ((M <= 2 || (M <= 8 && (N + 7) / 8 < 8 * sm_count())) && !w4a8_tile_only() && !w4a8_no_gemv()) {
-        w4a8::GemvArgs g{xq, a, xs, (const uint8_t*)wq, (const uint8_t*)wsc, (const uint8_t*)wmn, wd, wdm, out, ldo, n_rows, M, N,
-                         K, Ma, epi};
-        if (M == 1) return launch_w4a8_gemv<1>(kind, g, st);
-        if (M == 2) return launch_w4a8_gemv<2>(kind, g, st);
-        if (M <= 4) return launch_w4a8_gemv<4>(kind, g, st);
-        return launch_w4a8_gemv<8>(kind, g, st);
+    if (split > 1 && M > (N < 64 * sm_count() ? 8 : 2) && M <= 16 && !w4a8_tile_only()) {
+        // no kernel uses the workspace (K is split inside a CTA), but a caller's contract stays checked
+        if (!workspace || !counters) return PB_BAD_ARGUMENT;
+        if (workspace_bytes < pb_w4a8_workspace_bytes(M, N, K) || n_counters < pb_w4a8_counters(M, N)) return PB_TOO_LARGE;
     }
-    if (M <= 32 && !w4a8_tile_only()) {                            // measured: the many-rows kernel is faster from 64 rows
-        if (kind == 0) {
-            // K split (exact): Q4_K through tensor memory, one tile of 16 rows
-            if (split > 1 && M <= 16 && !w4a8_few_staged()) {
-                if (!workspace || !counters) return PB_BAD_ARGUMENT;
-                if (workspace_bytes < pb_w4a8_workspace_bytes(M, N, K) || n_counters < pb_w4a8_counters(M, N)) return PB_TOO_LARGE;
-            } else {
-                split = 1;
-            }
-            return launch_w4a8_few<w4a8::KIND_Q4K>(xq, a, xs, Ma, wq, wsc, wmn, wd, wdm, out, ldo, n_rows, M, N, K, epi, st,
-                                                   split, (float*)workspace, counters);
-        }
-        if (split > 1 && M <= 16) {
-            if (!workspace || !counters) return PB_BAD_ARGUMENT;
-            if (workspace_bytes < pb_w4a8_workspace_bytes(M, N, K) || n_counters < pb_w4a8_counters(M, N)) return PB_TOO_LARGE;
-        } else {
-            split = 1;
-        }
-        return launch_w4a8_few<w4a8::KIND_Q6K>(xq, a, xs, Ma, wq, wsc, wmn, wd, wdm, out, ldo, n_rows, M, N, K, epi, st,
-                                               split, (float*)workspace, counters);
+    // Up to 32 rows, or 64 against so few weight rows that the many-rows kernel's 64-column tiles leave most SMs idle (at
+    // 50 rows 12.9 against 29 us on 1024 rows of Q6_K, but 25 against 23 on 5120 of Q4_K).  One or two Q6_K rows stay on
+    // the CUDA cores (5120 x 17408: 20.5 / 22.4 us against 23.7; from four rows on 24.0 against 30.5).
+    if ((M <= 32 || (M <= 64 && N <= 16 * sm_count())) && !w4a8_tile_only()) {
+        const w4a8::GemvArgs g{xq, a, xs, (const uint8_t*)wq, (const uint8_t*)wsc, (const uint8_t*)wmn, wd, wdm, out, ldo, n_rows,
+                               M, N, K, Ma, epi};
+        if (kind == 0) return launch_w4a8_few<w4a8::KIND_Q4K>(g, st);
+        if (M <= 2 && N > 16 * sm_count() && !w4a8_no_gemv())
+            return M == 1 ? launch_w4a8_gemv<1>(g, st) : launch_w4a8_gemv<2>(g, st);
+        return launch_w4a8_few<w4a8::KIND_Q6K>(g, st);
     }
     if (kind == 0)
         return launch_w4a8<w4a8::KIND_Q4K>(xq, a, xs, Ma, wq, wsc, wmn, wd, wdm, out, ldo, n_rows, M, N, K, epi, st);

@@ -61,6 +61,32 @@ def test_gemm_bits(dev, kind, m, live, n, k):
     assert np.linalg.norm(got - true.numpy()) / np.linalg.norm(true.numpy()) < 0.05
 
 
+@pytest.mark.parametrize("kind", ["q4k", "q6k"])
+@pytest.mark.parametrize("m,live,n,k", [(3, 3, 20, 256), (9, 8, 36, 1280), (17, 17, 2500, 768), (31, 30, 68, 2304),
+                                        (33, 33, 1024, 512), (64, 64, 2052, 512), (8, 8, 18948, 512), (16, 13, 18948, 512),
+                                        (32, 32, 18948, 512)])
+def test_gemm_bits_decode_tiles(dev, kind, m, live, n, k):
+    """The decode kernels' edges: weight rows that end inside a tile of 16, 32 or 64, super-blocks that do not fill a round
+    of the warps, row counts just above a block of 8, 16 or 32, and both sides of the rule on the weight rows."""
+    g = torch.Generator().manual_seed(n + k + m)
+    u8 = lambda *s, hi: torch.randint(0, hi, s, generator=g, dtype=torch.uint8)          # noqa: E731
+    f = lambda: torch.rand(k // 256, n, generator=g) * 1e-3                              # noqa: E731
+    if kind == "q4k":
+        w = w4a8.W4(kind, u8(n, k // 2, hi=256), u8(k // 256, n, 8, hi=64), u8(k // 256, n, 8, hi=64), f(), f(), n, k)
+    else:
+        w = w4a8.W4(kind, torch.randint(-32, 32, (n, k), generator=g, dtype=torch.int8),
+                    torch.randint(-128, 128, (k // 256, n, 16), generator=g, dtype=torch.int8), None, f(), None, n, k)
+    xq, a, xs = oracle.quant_g(np_bits(synth.activations(m, k, seed=m, outliers=k // 64)))
+    base = torch.randn(m, n, generator=g)
+    ref0, ref1 = ref_gemm(xq, a, xs, w, 0, live), ref_gemm(xq, a, xs, w, 1, live, out=base.numpy().copy())
+    xqd, ad, xsd = (torch.from_numpy(t).to(dev) for t in (xq, a, xs))
+    out, res = torch.zeros(m, n, dtype=torch.bfloat16, device=dev), base.to(dev)
+    w4a8.gemm(xqd, ad, xsd, w.to(dev), out, n_rows(live, dev))
+    w4a8.gemm(xqd, ad, xsd, w.to(dev), res, n_rows(live, dev), epi=1)
+    assert same(out, bf16_from_bits(ref0)), first_diff(np_bits(out), ref0)
+    assert same(res, ref1), first_diff(res.cpu().numpy(), ref1)
+
+
 def test_fused_mixed_projection(dev):
     """q | k as Q4_K and v as Q6_K in one output buffer (the Q4_K_M convention), through rows_g on the GPU."""
     k, m = 1024, 20
