@@ -164,14 +164,12 @@ class LinearStack:
         M, nr, g = self.M, self.n_rows, self.g
         pend = None
         for lw in self.layers:
-            quant.fold(self.h, self.slots, pend, nr, M)
-            quant.rows_q8(self.h, None, self.xq, self.xs, nr, M)
+            quant.fold_rows_q8(self.h, self.slots, pend, self.xq, self.xs, nr, M)
             w8a8.gemm(self.xq, self.xs, *lw["qkv"], self.qkv, nr, self.hidden, pdl=self.pdl)
             tp.quantize_rows(g if self.n > 1 else None, quant.rows_q8, M, self.amax, self.qkv[:, :self.ql], None,
                              self.aq, self.as_, nr, M)
             pend = self._out(self.aq, self.as_, lw["o"])
-            quant.fold(self.h, self.slots, pend, nr, M)
-            quant.rows_q8(self.h, None, self.xq, self.xs, nr, M)
+            quant.fold_rows_q8(self.h, self.slots, pend, self.xq, self.xs, nr, M)
             w8a8.gemm(self.xq, self.xs, *lw["gate_up"], self.gu, nr, self.hidden, pdl=self.pdl)
             tp.quantize_rows(g if self.n > 1 else None, quant.swiglu_q8, M, self.amax, self.gu, None, self.dq,
                              self.ds, nr, M)

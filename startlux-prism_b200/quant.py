@@ -255,4 +255,25 @@ def fold(h, parts, pending, n, T):
         return
     rc = _lib.lib().pb_fold(_lib.ptr(h), h.stride(0), _lib.ptr(parts), parts.stride(0), pending.n,
                             _lib.ptr(pending.a_s), _lib.ptr(pending.w_s), _lib.ptr(n), T, N, _lib.stream())
-    _lib.check(rc, f"fold T={T} N={N} S={pending.n}")
+    if rc:
+        _lib.check(rc, f"fold T={T} N={N} S={pending.n}")
+
+
+def fold_rows_q8(h, parts, pending, q, s, n, T):
+    """fold(h, parts, pending, n, T) and then rows_q8(h, None, q, s, n, T): one launch when a deferred add of this rank's
+    own slots is pending (the same bits), otherwise the two calls."""
+    N = h.shape[1]
+    if not pending or pending.sync is not None or N % 8 or N > 65536:
+        fold(h, parts, pending, n, T)
+        return rows_q8(h, None, q, s, n, T)
+    if pending.parts is not None:
+        parts = pending.parts
+    _lib.need_cuda(h, parts, q, s, n)
+    if h.dtype != torch.float32 or parts.dtype != torch.int32 or parts.shape[2] != N or h.stride(1) != 1 \
+            or q.shape[1] != N or not q.is_contiguous():
+        raise RuntimeError("fold_rows_q8: h fp32 [T, N], parts int32 [S, rows, N], q int8 [T, N]")
+    rc = _lib.lib().pb_fold_rows_q8(_lib.ptr(h), h.stride(0), _lib.ptr(parts), parts.stride(0), pending.n,
+                                    _lib.ptr(pending.a_s), _lib.ptr(pending.w_s), _lib.ptr(q), _lib.ptr(s), _lib.ptr(n), T, N,
+                                    _lib.stream())
+    if rc:
+        _lib.check(rc, f"fold_rows_q8 T={T} N={N} S={pending.n}")

@@ -97,6 +97,24 @@ def test_fold_odd(dev):
     assert same(hd, ref)
 
 
+@pytest.mark.parametrize("T,N,S,live", [(1, 8, 1, 1), (16, 5120, 7, 13), (3, 8192, 2, 3), (5, 8200, 3, 5), (64, 264, 8, 64)])
+def test_fold_rows_q8(dev, T, N, S, live):
+    """The one-launch form against fold and rows_q8 of the oracle: residual, int8 rows and scales alike, rows >= live
+    untouched; either side of 8192 columns (one or eight vectors a thread), the scales written over the add's own."""
+    g = torch.Generator().manual_seed(N)
+    slots = torch.randint(-10 ** 6, 10 ** 6, (S, T, N), generator=g, dtype=torch.int32)
+    sa, sw = torch.rand(T, generator=g) * 1e-2, torch.rand(N, generator=g) * 1e-3
+    h = torch.randn(T, N, generator=g)
+    ref = oracle.fold(h.numpy().copy(), slots.numpy(), sa.numpy(), sw.numpy(), live=live)
+    rq, rs = oracle.quant_rows(ref, live=live)
+    hd, sd = h.to(dev), sa.to(dev)
+    q = torch.full((T, N), 99, dtype=torch.int8, device=dev)
+    quant.fold_rows_q8(hd, slots.to(dev), w8a8.Deferred(S, sd, sw.to(dev)), q, sd, n_rows(live, dev), T)
+    assert same(hd, ref)
+    assert same(q[:live], rq[:live]) and same(sd[:live], rs[:live, 0]) and same(sd[live:], sa[live:])
+    assert bool((q[live:] == 99).all())
+
+
 @pytest.mark.parametrize("T,K,live", [(300, 5120, 290), (1000, 2560, 1000), (260, 17408, 257), (512, 264, 512)])
 def test_rows_q8_many_rows(dev, T, K, live):
     """From 256 rows the row-pipelined kernel runs (persistent CTAs, rows staged in shared memory): the same bits as
