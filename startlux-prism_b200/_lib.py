@@ -113,7 +113,9 @@ def ptr(t):
 
 
 def stream():
-    return torch.cuda.current_stream().cuda_stream
+    """The current device's current stream as a raw handle (torch.cuda.current_stream().cuda_stream without building a
+    Stream object on every call)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def need_cuda(*tensors):

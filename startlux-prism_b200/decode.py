@@ -31,7 +31,8 @@ def head_quant(h, norm, q, s, n, B, eps):
         raise RuntimeError("head_quant: h fp32 [B, HID], q int8 [B, HID], s fp32 [B, HID / 32], contiguous")
     rc = _lib.lib().pb_head_quant(_lib.ptr(h), _lib.ptr(norm), _lib.ptr(q), _lib.ptr(s), _lib.ptr(n), B, HID, float(eps),
                                   _lib.stream())
-    _lib.check(rc, f"head_quant B={B} HID={HID}")
+    if rc:
+        _lib.check(rc, f"head_quant B={B} HID={HID}")
 
 
 def head_scales(w_s):

@@ -68,14 +68,16 @@ def push(src, dsts):
         raise RuntimeError("push: contiguous blocks of one size")
     arr = (ctypes.c_void_p * max(len(dsts), 1))(*[d.data_ptr() for d in dsts])
     rc = _lib.lib().pb_push(_lib.ptr(src), arr, len(dsts), src.numel() * src.element_size(), _lib.stream())
-    _lib.check(rc, f"push {src.numel() * src.element_size()} bytes to {len(dsts)} ranks")
+    if rc:
+        _lib.check(rc, f"push {src.numel() * src.element_size()} bytes to {len(dsts)} ranks")
 
 
 def handshake(sync):
     """The flag handshake of `sync` (tp.Group.handshake()) as a step of its own on the stream: signals every other rank
     and waits (bounded) for all of them."""
     rc = _lib.lib().pb_handshake(ctypes.byref(_sync_struct(sync)), _lib.stream())
-    _lib.check(rc, f"handshake over {sync.world} ranks")
+    if rc:
+        _lib.check(rc, f"handshake over {sync.world} ranks")
 
 
 def _mode_args(mode, amax, sync, T):
@@ -109,7 +111,8 @@ def rows_q8(x, inv_s, q, s, n, T, mode=0, amax=None, sync=None):
     else:
         rc = _lib.lib().pb_quant_rows(_lib.ptr(x), int(x.dtype == torch.float32), x.stride(0), _lib.ptr(inv_s),
                                       _lib.ptr(q), _lib.ptr(s), _lib.ptr(n), T, K, K, mode, _lib.ptr(amax), _lib.stream())
-    _lib.check(rc, f"rows_q8 T={T} K={K} mode={mode}")
+    if rc:
+        _lib.check(rc, f"rows_q8 T={T} K={K} mode={mode}")
 
 
 def swiglu_q8(gu, inv_s, q, s, n, T, mode=0, amax=None, sync=None):
@@ -125,7 +128,8 @@ def swiglu_q8(gu, inv_s, q, s, n, T, mode=0, amax=None, sync=None):
     else:
         rc = _lib.lib().pb_swiglu_q8(_lib.ptr(gu), _lib.ptr(inv_s), _lib.ptr(q), _lib.ptr(s), _lib.ptr(n), T, FF, mode,
                                      _lib.ptr(amax), _lib.stream())
-    _lib.check(rc, f"swiglu_q8 T={T} FF={FF} mode={mode}")
+    if rc:
+        _lib.check(rc, f"swiglu_q8 T={T} FF={FF} mode={mode}")
 
 
 def norm_q8(h, w_over_s, q, s, n, T, eps, rows=None, parts=None, pending=None):
@@ -146,13 +150,15 @@ def norm_q8(h, w_over_s, q, s, n, T, eps, rows=None, parts=None, pending=None):
         rc = _lib.lib().pb_norm_q8_sync(_lib.ptr(h), _lib.ptr(w_over_s), _lib.ptr(q), _lib.ptr(s), _lib.ptr(n), T, HID,
                                         float(eps), _lib.ptr(parts), parts.stride(0), np_, _lib.ptr(pending.a_s),
                                         _lib.ptr(pending.w_s), ctypes.byref(_sync_struct(pending.sync)), _lib.stream())
-        _lib.check(rc, f"norm_q8 T={T} HID={HID} parts={np_} over {pending.sync.world} ranks")
+        if rc:
+            _lib.check(rc, f"norm_q8 T={T} HID={HID} parts={np_} over {pending.sync.world} ranks")
         return
     rc = _lib.lib().pb_norm_q8(_lib.ptr(h), _lib.ptr(w_over_s), _lib.ptr(q), _lib.ptr(s), _lib.ptr(rows), _lib.ptr(n),
                                T, HID, float(eps), _lib.ptr(parts) if np_ else None, parts.stride(0) if np_ else 0, np_,
                                _lib.ptr(pending.a_s) if np_ else None, _lib.ptr(pending.w_s) if np_ else None,
                                _lib.stream())
-    _lib.check(rc, f"norm_q8 T={T} HID={HID} parts={np_}")
+    if rc:
+        _lib.check(rc, f"norm_q8 T={T} HID={HID} parts={np_}")
 
 
 def gated_norm_q8(o, proj, z_off, w, inv_s, q, s, n, T, cfg, mode=0, amax=None, sync=None):
@@ -174,7 +180,8 @@ def gated_norm_q8(o, proj, z_off, w, inv_s, q, s, n, T, cfg, mode=0, amax=None, 
         rc = _lib.lib().pb_gated_norm_q8(_lib.ptr(o), _lib.ptr(proj), proj.stride(0), int(z_off), _lib.ptr(w),
                                          _lib.ptr(inv_s), _lib.ptr(q), _lib.ptr(s), _lib.ptr(n), T, HV, D, float(cfg.eps),
                                          mode, _lib.ptr(amax), _lib.stream())
-    _lib.check(rc, f"gated_norm_q8 T={T} heads={HV} dim={D} mode={mode}")
+    if rc:
+        _lib.check(rc, f"gated_norm_q8 T={T} heads={HV} dim={D} mode={mode}")
 
 
 def rows_g(x, q, s, xs, n, T):
@@ -188,7 +195,8 @@ def rows_g(x, q, s, xs, n, T):
         raise RuntimeError("rows_g: s must be [K/256, M] and xs [K/256, M, 16], contiguous")
     rc = _lib.lib().pb_quant_g(_lib.ptr(x), int(x.dtype == torch.float32), _lib.ptr(q), _lib.ptr(s), _lib.ptr(xs),
                                _lib.ptr(n), T, Ma, K, _lib.stream())
-    _lib.check(rc, f"rows_g T={T} K={K}")
+    if rc:
+        _lib.check(rc, f"rows_g T={T} K={K}")
 
 
 def _g_outputs(q, s, xs, K, what):
@@ -208,7 +216,8 @@ def swiglu_g(gu, q, s, xs, n, T):
     if gu.dtype != torch.bfloat16 or gu.shape[1] != 2 * FF or not gu.is_contiguous():
         raise RuntimeError("swiglu_g: gu must be contiguous bf16 [T, 2 FF]")
     rc = _lib.lib().pb_swiglu_g(_lib.ptr(gu), _lib.ptr(q), _lib.ptr(s), _lib.ptr(xs), _lib.ptr(n), T, Ma, FF, _lib.stream())
-    _lib.check(rc, f"swiglu_g T={T} FF={FF}")
+    if rc:
+        _lib.check(rc, f"swiglu_g T={T} FF={FF}")
 
 
 def norm_g(h, w, q, s, xs, n, T, eps):
@@ -220,7 +229,8 @@ def norm_g(h, w, q, s, xs, n, T, eps):
         raise RuntimeError("norm_g: h must be contiguous fp32 [T, HID]")
     rc = _lib.lib().pb_norm_g(_lib.ptr(h), _lib.ptr(w), _lib.ptr(q), _lib.ptr(s), _lib.ptr(xs), _lib.ptr(n), T, Ma, HID,
                               float(eps), _lib.stream())
-    _lib.check(rc, f"norm_g T={T} HID={HID}")
+    if rc:
+        _lib.check(rc, f"norm_g T={T} HID={HID}")
 
 
 def gated_norm_g(o, proj, z_off, w, q, s, xs, n, T, cfg):
@@ -232,7 +242,8 @@ def gated_norm_g(o, proj, z_off, w, q, s, xs, n, T, cfg):
         raise RuntimeError("gated_norm_g: o fp32 contiguous, proj bf16 with unit column stride")
     rc = _lib.lib().pb_gated_norm_g(_lib.ptr(o), _lib.ptr(proj), proj.stride(0), int(z_off), _lib.ptr(w), _lib.ptr(q),
                                     _lib.ptr(s), _lib.ptr(xs), _lib.ptr(n), T, Ma, HV, D, float(cfg.eps), _lib.stream())
-    _lib.check(rc, f"gated_norm_g T={T} heads={HV} dim={D}")
+    if rc:
+        _lib.check(rc, f"gated_norm_g T={T} heads={HV} dim={D}")
 
 
 def fold(h, parts, pending, n, T):
@@ -251,7 +262,8 @@ def fold(h, parts, pending, n, T):
         rc = _lib.lib().pb_fold_sync(_lib.ptr(h), h.stride(0), _lib.ptr(parts), parts.stride(0), pending.n,
                                      _lib.ptr(pending.a_s), _lib.ptr(pending.w_s), _lib.ptr(n), T, N,
                                      ctypes.byref(_sync_struct(pending.sync)), _lib.stream())
-        _lib.check(rc, f"fold T={T} N={N} S={pending.n} over {pending.sync.world} ranks")
+        if rc:
+            _lib.check(rc, f"fold T={T} N={N} S={pending.n} over {pending.sync.world} ranks")
         return
     rc = _lib.lib().pb_fold(_lib.ptr(h), h.stride(0), _lib.ptr(parts), parts.stride(0), pending.n,
                             _lib.ptr(pending.a_s), _lib.ptr(pending.w_s), _lib.ptr(n), T, N, _lib.stream())

@@ -94,7 +94,7 @@ def pick_split(M, N, K, limit=MAX_SPLIT):
 _TABLE = None
 
 
-def _choice(M, N, K, residual):
+def _choice(M, N, K, residual, pdl=False):
     """The measured choice for this projection shape at the nearest measured row count (tune.py's table), or None."""
     global _TABLE
     if _TABLE is None:
@@ -104,8 +104,9 @@ def _choice(M, N, K, residual):
     if not by_m:
         return None
     import math
-    # the one-row entry was measured on the CUDA-core kernel: it says nothing about the tensor-core kernel at 2+ rows
-    rows = [x for x in by_m if x > GEMV_ROWS] if M > GEMV_ROWS else list(by_m)
+    # the one-row entry was measured on the CUDA-core kernel: it says nothing about the tensor-core kernel, which runs at
+    # two rows up and for a programmatic dependent of one row
+    rows = [x for x in by_m if x > GEMV_ROWS] if M > GEMV_ROWS or pdl else list(by_m)
     if not rows:
         return None
     m = min(rows, key=lambda x: abs(math.log(x) - math.log(max(M, 1))))
@@ -135,7 +136,8 @@ def _call(a, a_s, w, w_s, out, ldo, n_rows, gk, epi, split, slot_stride=0, ws=No
                                  _lib.ptr(n_rows), M, N, K, gk, epi, split, slot_stride, _lib.ptr(ws),
                                  0 if ws is None else ws.numel(), _lib.ptr(counters),
                                  0 if counters is None else counters.numel(), int(bool(pdl)), _lib.stream())
-    _lib.check(rc, f"w8a8 gemm M={M} N={N} K={K} gk={gk} epi={epi} split={split}")
+    if rc:
+        _lib.check(rc, f"w8a8 gemm M={M} N={N} K={K} gk={gk} epi={epi} split={split}")
 
 
 def _scales_ok(s, rows, groups, what):
@@ -181,7 +183,7 @@ def gemm(a, a_s, w, w_s, out, n_rows, gk, epi=0, outs=None, cfg=None, slots=None
     if cfg is not None:
         split = int(cfg)
     else:
-        c = _choice(M, N, K, epi == EPI_ADD) if M <= FEW_ROWS else None
+        c = _choice(M, N, K, epi == EPI_ADD, pdl) if M <= FEW_ROWS else None
         split = c["split"] if c else pick_split(M, N, K)
         defer_ok = c["defer"] if c else True
     split = effective_split(K, split)
@@ -226,7 +228,8 @@ def _gemm_swiglu(a, a_s, w, w_s, out, n_rows, gk, outs, cfg):
     _scales_ok(w_s, N, 1, "w_s")
     rc = _lib.lib().pb_w8a8_gemm_swiglu(_lib.ptr(a), _lib.ptr(a_s), _lib.ptr(w), _lib.ptr(w_s), _lib.ptr(out),
                                         out.stride(0), _lib.ptr(outs), _lib.ptr(n_rows), M, N, K, bn, _lib.stream())
-    _lib.check(rc, f"w8a8 gemm epi 2 M={M} N={N} K={K} bn={bn}")
+    if rc:
+        _lib.check(rc, f"w8a8 gemm epi 2 M={M} N={N} K={K} bn={bn}")
     return None
 
 
@@ -275,7 +278,8 @@ def gemm_scatter(a, w, blocks, block_rows, ldo, n_rows):
     arr = (ctypes.c_void_p * len(blocks))(*[int(b) for b in blocks])
     rc = _lib.lib().pb_w8a8_gemm_scatter(_lib.ptr(a), _lib.ptr(w), arr, len(blocks), block_rows, ldo, _lib.ptr(n_rows),
                                          M, N, K, _lib.stream())
-    _lib.check(rc, f"w8a8 gemm_scatter M={M} N={N} K={K} blocks={len(blocks)}x{block_rows}")
+    if rc:
+        _lib.check(rc, f"w8a8 gemm_scatter M={M} N={N} K={K} blocks={len(blocks)}x{block_rows}")
 
 
 def quant_rows(x, gk, n_rows=None):
@@ -290,7 +294,8 @@ def quant_rows(x, gk, n_rows=None):
         raise RuntimeError("quant_rows: x must be contiguous bf16 or fp32")
     rc = _lib.lib().pb_quant_rows(_lib.ptr(x), int(x.dtype == torch.float32), K, None, _lib.ptr(q), _lib.ptr(s),
                                   _lib.ptr(n_rows), M, K, gk, 0, None, _lib.stream())
-    _lib.check(rc, f"quant_rows M={M} K={K} gk={gk}")
+    if rc:
+        _lib.check(rc, f"quant_rows M={M} K={K} gk={gk}")
     return q, s
 
 
