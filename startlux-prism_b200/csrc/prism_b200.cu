@@ -1065,6 +1065,22 @@ int pb_fold(float* h, long ldh, const int32_t* slots, long slot_stride, int S, c
     return PB_OK;
 }
 
+int pb_fold_rows_q8(float* h, long ldh, const int32_t* slots, long slot_stride, int S, const float* a_s, const float* w_s,
+                    int8_t* q, float* s, const int* n_rows, int rows, int N, void* stream) {
+    if (!h || !slots || !a_s || !w_s || !q || !s || !n_rows || rows <= 0 || N <= 0 || S < 1 || ldh < N) return PB_BAD_ARGUMENT;
+    if (N % 8 || N > 65536) return PB_UNSUPPORTED_SHAPE;
+    if (!aligned16(h) || !aligned16(slots) || !aligned16(w_s) || ((uintptr_t)q & 7) || ldh % 4 || slot_stride % 4)
+        return PB_BAD_ARGUMENT;
+    const int nvec = N / 8, vpt = nvec <= 1024 ? 1 : 8;
+    const int threads = ((nvec + vpt - 1) / vpt + 31) / 32 * 32;
+    auto kern = div_full() ? (vpt == 1 ? quant::fold_rows_q8_kernel<1, true> : quant::fold_rows_q8_kernel<8, true>)
+                           : (vpt == 1 ? quant::fold_rows_q8_kernel<1, false> : quant::fold_rows_q8_kernel<8, false>);
+    PB_CUDA(launch_dep(kern, dim3(rows), dim3(threads), 0, (cudaStream_t)stream, h, ldh, slots, slot_stride, S, a_s, w_s, q, s,
+                       n_rows, N));
+    PB_CUDA(cudaGetLastError());
+    return PB_OK;
+}
+
 // pb_sync (the C struct) -> the kernels' view; world <= 1 when there is none
 static int to_sync(const pb_sync* in, tpx::Sync* out, bool need_others) {
     memset(out, 0, sizeof(*out));
@@ -1104,22 +1120,6 @@ static int quant_rows_impl(const void* x, int x_fp32, long ldx, const float* inv
         } else {
             if (full) quant::quant_groups_kernel<false, true><<<grid, 256, 0, st>>>(x, q, s, n_rows, K, gk);
             else quant::quant_groups_kernel<false, false><<<grid, 256, 0, st>>>(x, q, s, n_rows, K, gk);
-int pb_fold_rows_q8(float* h, long ldh, const int32_t* slots, long slot_stride, int S, const float* a_s, const float* w_s,
-                    int8_t* q, float* s, const int* n_rows, int rows, int N, void* stream) {
-    if (!h || !slots || !a_s || !w_s || !q || !s || !n_rows || rows <= 0 || N <= 0 || S < 1 || ldh < N) return PB_BAD_ARGUMENT;
-    if (N % 8 || N > 65536) return PB_UNSUPPORTED_SHAPE;
-    if (!aligned16(h) || !aligned16(slots) || !aligned16(w_s) || ((uintptr_t)q & 7) || ldh % 4 || slot_stride % 4)
-        return PB_BAD_ARGUMENT;
-    const int nvec = N / 8, vpt = nvec <= 1024 ? 1 : 8;
-    const int threads = ((nvec + vpt - 1) / vpt + 31) / 32 * 32;
-    auto kern = div_full() ? (vpt == 1 ? quant::fold_rows_q8_kernel<1, true> : quant::fold_rows_q8_kernel<8, true>)
-                           : (vpt == 1 ? quant::fold_rows_q8_kernel<1, false> : quant::fold_rows_q8_kernel<8, false>);
-    PB_CUDA(launch_dep(kern, dim3(rows), dim3(threads), 0, (cudaStream_t)stream, h, ldh, slots, slot_stride, S, a_s, w_s, q, s,
-                       n_rows, N));
-    PB_CUDA(cudaGetLastError());
-    return PB_OK;
-}
-
         }
         PB_CUDA(cudaGetLastError());
         return PB_OK;
