@@ -17,6 +17,7 @@
 #include "w8a8_gemm.cuh"
 #include "w8a8_groups.cuh"
 #include "w8a8_g32.cuh"
+#include "w8a8_g32_mma.cuh"
 #include "w4a8_gemm.cuh"
 #include "w4a8_gemv.cuh"
 #include "w4a8_mma.cuh"
@@ -434,24 +435,21 @@ int grouped_rows_per_cta(int M, int N) {
     return 16;
 }
 
-// Per-32 groups, one K slice (w8a8_g32.cuh): NB = 16 with row blocks of 16, 8 or 4 per CTA, or NB = 32 (more than 16 rows).
-template <int NB, int RW>
+// Per-32 groups, one K slice, on tcgen05 (w8a8_g32.cuh): row blocks of 16.
 int launch_g32(const int8_t* a, const int8_t* w, w8a8::SwapArgs p, cudaStream_t st) {
-    using C = w8a8::G32<NB>;
-    constexpr int RCTA = 2 * RW;
+    using C = w8a8::G32;
     CUtensorMap tw, tx;
     int rc;
     if ((rc = tensor_map_kchunks(&tw, w, p.N, p.K, w8a8::BM))) return rc;
-    if ((rc = tensor_map_kchunks(&tx, a, p.M, p.K, NB))) return rc;
-    p.stages = C::stages_for(p.K, RCTA);
-    const int smem = C::smem_bytes(p.K, RCTA, p.stages);
-    auto kern = w8a8::w8a8_g32_kernel<NB, RW>;
+    if ((rc = tensor_map_kchunks(&tx, a, p.M, p.K, C::NB))) return rc;
+    p.stages = C::stages_for(p.K);
+    auto kern = w8a8::w8a8_g32_kernel;
     if ((rc = set_smem(kern, 232448))) return rc;
-    dim3 grid((p.N + w8a8::BM - 1) / w8a8::BM, 1, (p.M + RCTA - 1) / RCTA);
+    dim3 grid((p.N + w8a8::BM - 1) / w8a8::BM, 1, (p.M + C::NB - 1) / C::NB);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(C::THREADS);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = C::smem_bytes(p.K, p.stages);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -462,31 +460,72 @@ int launch_g32(const int8_t* a, const int8_t* w, w8a8::SwapArgs p, cudaStream_t 
     return PB_OK;
 }
 
-// Can w8a8_g32_kernel take the call?  One K slice, a direct store, and room for at least three stages beside the
-// activation scales (K up to about 80 k at 16 rows, 40 k at 32).  PRISM_B200_G32=0 keeps the older kernel (comparisons).
-int g32_rows(const w8a8::SwapArgs& p, int split) {
+// The same on mma.sync (w8a8_g32_mma.cuh): 8 * MT * WM activation rows x 16 * NT * WN weight rows per CTA.
+template <int MT, int NT, int WN, int WM, int KQ, int ST>
+int launch_g32_mma(const int8_t* a, const int8_t* w, const w8a8::SwapArgs& p, cudaStream_t st) {
+    using C = w8a8::G32Mma<MT, NT, WN, WM, KQ, ST>;
+    static_assert(C::SMEM <= 232448, "shared memory of a CTA");
+    auto kern = p.epi == w8a8::EPI_F32 ? w8a8::w8a8_g32_mma_kernel<MT, NT, WN, WM, KQ, ST, true>
+                                       : w8a8::w8a8_g32_mma_kernel<MT, NT, WN, WM, KQ, ST, false>;
+    int rc;
+    if ((rc = set_smem(kern, C::SMEM))) return rc;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((p.M + C::MC - 1) / C::MC) * (unsigned)((p.N + C::ROWS - 1) / C::ROWS));
+    cfg.blockDim = dim3(C::THREADS);
+    cfg.dynamicSmemBytes = C::SMEM;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = p.pdl ? 1 : 0;
+    PB_CUDA(cudaLaunchKernelEx(&cfg, kern, a, w, p));
+    return PB_OK;
+}
+
+// Which one (measured: 5120 / 7168 / 34816 x 5120, 5120 x 17408 and the 248320 x 5120 head, 1 to 1000 rows).
+//   - 17 rows up, while row blocks of 16 against 128-row weight tiles fit one wave: tcgen05, whose CTAs then spread the chain
+//     over more SMs than warps of 16 weight rows do (5120 x 5120 at 32 rows: 18.9 us against 19.8).
+//   - up to 16 rows: one warp per 16 weight rows x 8 rows in a CTA of its own, so that a few weight rows still cover the SMs
+//     (5120 x 5120: 11.0 / 12.5 us at 8 / 16 rows; 13.8 and 18.5 in CTAs of four); with N / 16 warps eight per SM already,
+//     CTAs that share the activations (34816 rows, 16 rows: 39.0 us against 50.5).
+//   - more: warps of 32 weight rows, whose two tiles share every activation operand and scale read from shared memory -
+//     its bandwidth is the bound at one tile per warp (head at 48 rows: 379 us against 418) - on CTA tiles of 64 x 64, 64 x 48
+//     or 128 x 24, whichever leaves the least idle in the last round of CTAs per SM.
+int launch_g32_any(const int8_t* a, const int8_t* w, const w8a8::SwapArgs& p, cudaStream_t st) {
+    const int M = p.M, N = p.N;
+    const long sms = sm_count();
+    const bool wide = N >= 16 * 8 * sms;
+    if (M > 16 && (long)((N + 127) / 128) * ((M + 15) / 16) <= sms && w8a8::G32::stages_for(p.K) >= 3)
+        return launch_g32(a, w, p, st);
+    if (M <= 8) return wide ? launch_g32_mma<1, 1, 2, 1, 2, 4>(a, w, p, st) : launch_g32_mma<1, 1, 1, 1, 4, 3>(a, w, p, st);
+    if (M <= 16) {
+        if (!wide) return launch_g32_mma<1, 1, 1, 2, 4, 3>(a, w, p, st);
+        return N >= 64 * 8 * sms ? launch_g32_mma<2, 2, 2, 1, 2, 3>(a, w, p, st) : launch_g32_mma<2, 2, 4, 1, 1, 3>(a, w, p, st);
+    }
+    if (M <= 64 && !wide) return launch_g32_mma<2, 1, 2, 2, 2, 4>(a, w, p, st);
+    if (M <= 32) return launch_g32_mma<4, 2, 4, 1, 1, 3>(a, w, p, st);
+    if (M <= 48) return launch_g32_mma<6, 2, 4, 1, 1, 3>(a, w, p, st);
+    // rounds of CTAs per SM x the tile's 16 x 8 units x its measured time per unit
+    const auto cost = [&](int rows, int mc, int time) {
+        return ((long)((N + rows - 1) / rows) * ((M + mc - 1) / mc) + sms - 1) / sms * (rows / 16) * (mc / 8) * time;
+    };
+    const long c64 = cost(64, 64, 68), c48 = cost(64, 48, 68), c24 = cost(128, 24, 72);
+    if (c64 <= c48 && c64 <= c24) return launch_g32_mma<4, 2, 2, 2, 1, 4>(a, w, p, st);
+    return c48 <= c24 ? launch_g32_mma<3, 2, 2, 2, 1, 4>(a, w, p, st) : launch_g32_mma<3, 2, 4, 1, 1, 3>(a, w, p, st);
+}
+
+// Can those kernels take the call?  One K slice and a direct store.  PRISM_B200_G32=0 keeps the older kernel (comparisons).
+bool g32_direct(const w8a8::SwapArgs& p, int split) {
     static const bool on = [] { const char* e = getenv("PRISM_B200_G32"); return !(e && e[0] == '0'); }();
-    if (!on || split != 1 || p.mode != w8a8::MODE_DIRECT || p.wrows != 0 || p.K % 128 != 0 ||
-        !(p.epi == w8a8::EPI_BF16 || p.epi == w8a8::EPI_ADD || p.epi == w8a8::EPI_F32))
-        return 0;
-    // more than 16 rows: row blocks of 16 while they all fit one wave (the per-group fp32 chain, which bounds the kernel,
-    // then spreads over more SMs: 20 against 31 us on 5120 x 5120 at 32 rows), blocks of 32 beyond that (half the
-    // re-reads of the weights from L2: 31.6 against 37.8 us at 64 rows)
-    const long blocks16 = (long)((p.N + 127) / 128) * ((p.M + 15) / 16);
-    if (p.M > 16 && blocks16 > sm_count() && w8a8::G32<32>::stages_for(p.K, 32) >= 3) return 32;
-    return w8a8::G32<16>::stages_for(p.K, 16) >= 3 ? 16 : 0;
+    return on && split == 1 && p.mode == w8a8::MODE_DIRECT && p.wrows == 0 && p.K % 128 == 0 &&
+           (p.epi == w8a8::EPI_BF16 || p.epi == w8a8::EPI_ADD || p.epi == w8a8::EPI_F32);
 }
 
 template <bool GROUPED>
 int launch_swap_nb(int nb, const int8_t* a, const float* a_s, const int8_t* w, const float* w_s, w8a8::SwapArgs p,
                    int split, cudaStream_t st) {
-    if constexpr (GROUPED) if (const int rows = g32_rows(p, split)) {
-        if (rows == 32) return launch_g32<32, 16>(a, w, p, st);
-        const int r = p.M <= 16 ? grouped_rows_per_cta(p.M, p.N) : 16;
-        if (r == 4) return launch_g32<16, 2>(a, w, p, st);
-        if (r == 8) return launch_g32<16, 4>(a, w, p, st);
-        return launch_g32<16, 8>(a, w, p, st);
-    }
+    if constexpr (GROUPED) if (g32_direct(p, split)) return launch_g32_any(a, w, p, st);
     if constexpr (GROUPED) if (nb == 16 && split == 1) {
         const int r = grouped_rows_per_cta(p.M, p.N);
         if (r == 4) return launch_swap<16, GROUPED, 2>(a, a_s, w, w_s, p, split, st);

@@ -337,3 +337,28 @@ def test_l2_prefetch(dev):
     assert same(out, bf16_from_bits(ref0))
     with pytest.raises(RuntimeError):
         w8a8.l2_prefetch([])
+
+
+@pytest.mark.parametrize("M,N,K,live", [(3, 20, 128, 3), (9, 33, 384, 8), (30, 1000, 640, 30), (50, 200, 256, 49),
+                                        (8, 18945, 256, 7), (16, 18960, 128, 16), (16, 75800, 128, 15), (17, 19000, 128, 17),
+                                        (33, 19000, 128, 33), (64, 19000, 128, 60), (65, 130, 384, 65), (500, 7168, 256, 499),
+                                        (256, 34816, 128, 256)])
+def test_groups_of_32_every_tile(dev, M, N, K, live):
+    """Per-32 groups on every CTA tile of the dispatch (each side of its lines in M and N), weight rows that end inside a
+    tile, pieces of K that do not fill a pipeline stage, live < M: the oracle's bits; rows >= live untouched."""
+    a, w, sa, sw = rand_w8a8(M, N, K, seed=M + N, groups=K // 32)
+    args = (a.numpy(), sa.numpy(), w.numpy(), sw.numpy(), 32)
+    dargs = (a.to(dev), sa.to(dev), w.to(dev), sw.to(dev))
+    out = torch.zeros(M, N, dtype=torch.bfloat16, device=dev)
+    w8a8.gemm(*dargs, out, n_rows(live, dev), 32)
+    ref = oracle.w8a8_gemm(*args, 0, live)
+    assert np.array_equal(np_bits(out)[:live], ref[:live]), first_diff(np_bits(out)[:live], ref[:live])
+    h0 = torch.randn(M, N, generator=torch.Generator().manual_seed(M))
+    h = h0.to(dev)
+    w8a8.gemm(*dargs, h, n_rows(live, dev), 32, epi=1)
+    assert same(h, oracle.w8a8_gemm(*args, 1, live, out=h0.numpy().copy()))
+    if M <= 64:                                           # the head's plain fp32 store and fused chain
+        f = torch.full((M, N), 7.0, device=dev)
+        w8a8.gemm(*dargs, f, n_rows(live, dev), 32, epi=w8a8.EPI_F32)
+        ref = oracle.w8a8_gemm(*args, 4, live)
+        assert np.array_equal(f.cpu().numpy()[:live], ref[:live]) and bool((f[live:] == 7.0).all())
