@@ -582,7 +582,7 @@ int launch_w4a8(const int8_t* xq, const float* a, const int8_t* xs, int Ma, cons
     if ((rc = set_smem(kern, C::SMEM))) return rc;
     w4a8::Args p{a, out, ldo, n_rows, M, N, K, Ma, epi};
     const int grid = ((M + 127) / 128) * ((N + 63) / 64);
-    kern<<<grid, w4a8::THREADS, C::SMEM, st>>>(m, p);
+    kern<<<grid, C::THREADS, C::SMEM, st>>>(m, p);
     PB_CUDA(cudaGetLastError());
     return PB_OK;
 }

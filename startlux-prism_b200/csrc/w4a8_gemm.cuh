@@ -13,8 +13,9 @@
 // and Q4_K's mins are one more K = 32 MMA per super-block: A = the activation group sums (eight S & 63, eight S >> 6,
 // as the quantizer stores them), B = the 6-bit mins placed against the low or the high parts: mins = MLO + 64 MHI.
 //
-// One CTA per 128 x 64 output tile; warps: 0 TMA producer, 1 MMA issuer, 2-5 expanders (packed weights -> int8 planes
-// in the 128-byte-swizzled operand layout), 6-13 epilogue (two per tensor-memory lane quarter: 32 columns each).  Per
+// One CTA per 128 x 64 output tile; warps: 0 TMA producer, 1 and the last one MMA issuers, four or eight expanders (packed
+// weights -> int8 planes in the 128-byte-swizzled operand layout), eight epilogue (two per tensor-memory lane quarter: 32
+// columns each).  Per
 // super-block the MMAs fill one of two accumulator sets in tensor memory while the epilogue warps drain the other
 // (the floating-point step per 256 inputs).
 #pragma once
@@ -24,7 +25,6 @@ namespace w4a8 {
 
 constexpr int BM = 128, BN = 64;
 constexpr int KIND_Q4K = 0, KIND_Q6K = 1;
-constexpr int THREADS = 15 * 32;               // producer, MMA issuer, 4 expanders, 8 epilogue warps, second MMA issuer
 
 template <int KIND>
 struct Cfg {
@@ -40,6 +40,12 @@ struct Cfg {
     static constexpr int TX_BYTES = OFF_MN + MN_BYTES;
     static constexpr int STAGE_BYTES = (TX_BYTES + 1023) / 1024 * 1024;
     static constexpr int STAGES = 3;
+    // Expander warps.  Q6_K's split of a product into two planes is about four times Q4_K's work per weight byte, and with four
+    // warps it was the slowest role: eight take 5120 x 17408 at 2048 rows from 744 to 606 us and at 128 rows from 88 to 73.
+    // Q4_K keeps four (34816 x 5120 at 2048 rows: 1,240 us against 1,263 with eight, whose threads leave fewer registers).
+    static constexpr int EXPW = KIND == KIND_Q4K ? 4 : 8;
+    static constexpr int EPI0 = 2 + EXPW;                                // first epilogue warp
+    static constexpr int THREADS = (EPI0 + 8 + 1) * 32;                  // producer, MMA issuer, expanders, 8 epilogue, second MMA issuer
     static constexpr int BX_BYTES = 2 * 128 * 128;                       // expanded planes: two K blocks x 128 rows
     static constexpr int BM_BYTES = KIND == KIND_Q4K ? 128 * 16 : 0;     // mins operand (one 16-byte K chunk per row)
     static constexpr int EXP_BYTES = BX_BYTES + 2048;
@@ -116,7 +122,7 @@ __device__ __forceinline__ void split_q6(uint32_t w, int sc, uint32_t kc, uint32
 }
 
 template <int KIND>
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(Cfg<KIND>::THREADS, 1)
 w4a8_kernel(const __grid_constant__ Maps maps, const Args p) {
     using C = Cfg<KIND>;
     extern __shared__ uint8_t smem_raw[];
@@ -134,14 +140,14 @@ w4a8_kernel(const __grid_constant__ Maps maps, const Args p) {
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::STAGES; ++s) {
             mbar_init(smem_u32(&aux->full[s]), 1);
-            mbar_init(smem_u32(&aux->empty[s]), 1 + 4);                  // MMA commit, expander warps
+            mbar_init(smem_u32(&aux->empty[s]), 1 + C::EXPW);            // MMA commit, expander warps
         }
         for (int i = 0; i < C::SCL_SLOTS; ++i) {
             mbar_init(smem_u32(&aux->sfull[i]), 1);
             mbar_init(smem_u32(&aux->sempty[i]), 8);                     // the 8 epilogue warps
         }
         for (int e = 0; e < 2; ++e) {
-            mbar_init(smem_u32(&aux->exp_full[e]), 4);
+            mbar_init(smem_u32(&aux->exp_full[e]), C::EXPW);
             mbar_init(smem_u32(&aux->exp_empty[e]), 1);
             mbar_init(smem_u32(&aux->acc_full[e]), 1);
             mbar_init(smem_u32(&aux->acc_empty[e]), 8);
@@ -149,7 +155,7 @@ w4a8_kernel(const __grid_constant__ Maps maps, const Args p) {
         aux->abort_flag = 0;
         mbar_fence_init();
     }
-    for (int i = threadIdx.x; i < 2048 / 16; i += THREADS) *(uint4*)(smem + C::OFF_ZERO + i * 16) = make_uint4(0, 0, 0, 0);
+    for (int i = threadIdx.x; i < 2048 / 16; i += C::THREADS) *(uint4*)(smem + C::OFF_ZERO + i * 16) = make_uint4(0, 0, 0, 0);
     if (warp == 1) {
         tmem_alloc(smem_u32(&aux->tmem_base), C::TMEM_COLS);
         tmem_relinquish();
@@ -211,9 +217,9 @@ w4a8_kernel(const __grid_constant__ Maps maps, const Args p) {
                 }
             }
         }
-    } else if (warp == 1 || warp == 14) {
+    } else if (warp == 1 || warp == C::EPI0 + 8) {
         // ------------------------------------------------------------------ MMA issuers
-        // Two threads take alternate super-blocks (warp 1 the even ones, warp 14 the odd ones): one thread's iteration -
+        // Two threads take alternate super-blocks (warp 1 the even ones, the last warp the odd ones): one thread's iteration -
         // three barrier waits, nine MMAs, three commits - takes about 1,000 cycles (cycle stamps on a B200) against 580
         // of MMA time.  Super-block b uses accumulator set and operand buffer b & 1, so each thread owns one of each and
         // every set is started (accumulate = 0) and committed by the thread that issues all of its MMAs.
@@ -249,10 +255,12 @@ w4a8_kernel(const __grid_constant__ Maps maps, const Args p) {
                 tc_commit(smem_u32(&aux->acc_full[e]));
             }
         }
-    } else if (warp < 6) {
+    } else if (warp < C::EPI0) {
         // ------------------------------------------------------------------ expanders: packed weights -> int8 planes
         const int t = threadIdx.x - 64;
-        const int n = t & 63, h = t >> 6;                                // weight row in the tile, K half
+        constexpr int PARTS = C::EXPW / 2;                               // threads per weight row
+        const int n = t & 63, part = t >> 6;                             // weight row in the tile, share of its 256 inputs:
+        const int h = part * 2 / PARTS, sub = part % (PARTS / 2);        // K half, share of the half
         int stage = 0;
         uint32_t phase = 0;
         for (int b = 0; b < NSB; ++b) {
@@ -268,19 +276,21 @@ w4a8_kernel(const __grid_constant__ Maps maps, const Args p) {
                 const uint2 sc8 = *(const uint2*)(st + C::OFF_SC + n * 8);
                 const uint32_t scw = h == 0 ? sc8.x : sc8.y;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
+                for (int jj = 0; jj < 8 / PARTS; ++jj) {
+                    const int j = sub * (8 / PARTS) + jj;
                     const uint4 w = *(const uint4*)(wq + swz(n, h * 4 + j));
                     expand_q4(bx, n, j, w, (scw >> (8 * j)) & 0xff);
                 }
                 const uint2 mn8 = *(const uint2*)(st + C::OFF_MN + n * 8);
                 uint8_t* bm = ex + C::BX_BYTES;
-                if (h == 0) *(uint4*)(bm + n * 16) = make_uint4(mn8.x, mn8.y, 0, 0);
-                else *(uint4*)(bm + (64 + n) * 16) = make_uint4(0, 0, mn8.x, mn8.y);
+                if (sub == 0 && h == 0) *(uint4*)(bm + n * 16) = make_uint4(mn8.x, mn8.y, 0, 0);
+                if (sub == 0 && h == 1) *(uint4*)(bm + (64 + n) * 16) = make_uint4(0, 0, mn8.x, mn8.y);
             } else {
                 const uint8_t* wq = st + C::OFF_WQ + h * BN * 128;       // this K half: 64 rows x 128 bytes, swizzled
                 const uint2 sc8 = *(const uint2*)(st + C::OFF_SC + n * 16 + h * 8);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
+                for (int ii = 0; ii < 16 / PARTS; ++ii) {
+                    const int i = sub * (16 / PARTS) + ii;
                     const int sc = (int)(int8_t)(((i < 4 ? sc8.x : sc8.y) >> (8 * (i & 3))) & 0xff);
                     const uint32_t kc = (uint32_t)(4096 - 32 * sc) * 0x00010001u;
                     const uint4 w = *(const uint4*)(wq + swz(n, i));
@@ -306,7 +316,7 @@ w4a8_kernel(const __grid_constant__ Maps maps, const Args p) {
         }
     } else {
         // ------------------------------------------------------------------ epilogue: 8 warps, 32 rows x 32 columns each
-        const int q = warp & 3, ch = (warp - 6) >> 2;
+        const int q = warp & 3, ch = (warp - C::EPI0) >> 2;
         const int ml = q * 32 + lane;                                    // row in the tile
         const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16) + ch * 32;
         // two output columns per instruction (packed fp32 multiply and fused multiply-add: each half rounds like its
@@ -334,17 +344,17 @@ w4a8_kernel(const __grid_constant__ Maps maps, const Args p) {
             tc_fence_after();
             const uint32_t set = lane_base + e * C::SET_COLS;
 #pragma unroll
-            for (int c = 0; c < 32; c += 16) {
-                uint32_t p0[16], p1[16];
-                tmem_ld16(set + c, p0);
-                tmem_ld16(set + 64 + c, p1);
+            for (int c = 0; c < 32; c += 8) {                            // eight columns at a time: registers for 19 warps
+                uint32_t p0[8], p1[8];
+                tmem_ld8(set + c, p0);
+                tmem_ld8(set + 64 + c, p1);
                 if (KIND == KIND_Q4K) {
-                    uint32_t l0[16], l1[16];
-                    tmem_ld16(set + 128 + c, l0);
-                    tmem_ld16(set + 192 + c, l1);
+                    uint32_t l0[8], l1[8];
+                    tmem_ld8(set + 128 + c, l0);
+                    tmem_ld8(set + 192 + c, l1);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 16; j += 2) {
+                    for (int j = 0; j < 8; j += 2) {
                         const float2 fa = make_float2(__int2float_rn((int)p0[j] + 8 * (int)p1[j]),
                                                       __int2float_rn((int)p0[j + 1] + 8 * (int)p1[j + 1]));
                         const float2 fm = make_float2(__int2float_rn((int)l0[j] + 64 * (int)l1[j]),
@@ -357,7 +367,7 @@ w4a8_kernel(const __grid_constant__ Maps maps, const Args p) {
                 } else {
                     tmem_ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 16; j += 2) {
+                    for (int j = 0; j < 8; j += 2) {
                         const float2 fa = make_float2(__int2float_rn((int)p0[j] + 64 * (int)p1[j]),
                                                       __int2float_rn((int)p0[j + 1] + 64 * (int)p1[j + 1]));
                         y2[(c + j) >> 1] = __ffma2_rn(am2, __fmul2_rn(dv[(c + j) >> 1], fa), y2[(c + j) >> 1]);
@@ -380,7 +390,7 @@ w4a8_kernel(const __grid_constant__ Maps maps, const Args p) {
         if (ok) {
             // every MMA has completed (the last accumulator set was full): the expanded-operand buffers are free and
             // serve as the transpose staging of the coalesced store (32 rows x 33 words per warp)
-            uint32_t* stg = (uint32_t*)(smem + C::OFF_EXP) + (warp - 6) * (32 * 33);
+            uint32_t* stg = (uint32_t*)(smem + C::OFF_EXP) + (warp - C::EPI0) * (32 * 33);
             const int rows_here = live - (m0 + q * 32);
             const int ncol0 = n0 + ch * 32;
             if (p.epi == 0) {
