@@ -435,21 +435,22 @@ int grouped_rows_per_cta(int M, int N) {
     return 16;
 }
 
-// Per-32 groups, one K slice, on tcgen05 (w8a8_g32.cuh): row blocks of 16.
+// Per-32 groups, one K slice, on tcgen05 (w8a8_g32.cuh): row blocks of NB = 16 or 32.
+template <int NB>
 int launch_g32(const int8_t* a, const int8_t* w, w8a8::SwapArgs p, cudaStream_t st) {
-    using C = w8a8::G32;
+    using C = w8a8::G32<NB>;
     CUtensorMap tw, tx;
     int rc;
     if ((rc = tensor_map_kchunks(&tw, w, p.N, p.K, w8a8::BM))) return rc;
-    if ((rc = tensor_map_kchunks(&tx, a, p.M, p.K, C::NB))) return rc;
-    p.stages = C::stages_for(p.K);
-    auto kern = w8a8::w8a8_g32_kernel;
+    if ((rc = tensor_map_kchunks(&tx, a, p.M, p.K, NB))) return rc;
+    p.stages = C::stages_for(p.K, NB);
+    auto kern = w8a8::w8a8_g32_kernel<NB, NB / 2>;
     if ((rc = set_smem(kern, 232448))) return rc;
-    dim3 grid((p.N + w8a8::BM - 1) / w8a8::BM, 1, (p.M + C::NB - 1) / C::NB);
+    dim3 grid((p.N + w8a8::BM - 1) / w8a8::BM, 1, (p.M + NB - 1) / NB);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(C::THREADS);
-    cfg.dynamicSmemBytes = C::smem_bytes(p.K, p.stages);
+    cfg.dynamicSmemBytes = C::smem_bytes(p.K, NB, p.stages);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -483,27 +484,35 @@ int launch_g32_mma(const int8_t* a, const int8_t* w, const w8a8::SwapArgs& p, cu
     return PB_OK;
 }
 
-// Which one (measured: 5120 / 7168 / 34816 x 5120, 5120 x 17408 and the 248320 x 5120 head, 1 to 1000 rows).
-//   - 17 rows up, while row blocks of 16 against 128-row weight tiles fit one wave: tcgen05, whose CTAs then spread the chain
-//     over more SMs than warps of 16 weight rows do (5120 x 5120 at 32 rows: 18.9 us against 19.8).
+// Which one (measured at 1 to 1000 rows on 1792 ... 34816 x 5120, 5120 x 8704 / 17408 and the 248320 x 5120 head; us, tcgen05
+// against mma.sync).
 //   - up to 16 rows: one warp per 16 weight rows x 8 rows in a CTA of its own, so that a few weight rows still cover the SMs
-//     (5120 x 5120: 11.0 / 12.5 us at 8 / 16 rows; 13.8 and 18.5 in CTAs of four); with N / 16 warps eight per SM already,
-//     CTAs that share the activations (34816 rows, 16 rows: 39.0 us against 50.5).
-//   - more: warps of 32 weight rows, whose two tiles share every activation operand and scale read from shared memory -
+//     (5120 x 5120: 12.8 against 11.1 at 8 rows, 13.5 against 12.1 at 12); with N / 16 warps eight per SM already (`wide`), CTAs that
+//     share the activations (34816 rows, 16 rows: 39.0 us against 50.5 without).  Between them, where the 128-row tiles of
+//     tcgen05 alone are one nearly full wave, that kernel (17408 rows, 12 rows: 21.7 against 26.8).
+//   - 17 to 64 rows, not wide: tcgen05 in row blocks of 16 while they fit one wave (5120 x 5120 at 24 rows 18.9 against 19.8), else
+//     of 32 (7168 at 40 rows 30.1 against 35.5); at 33 rows up against few weight rows warps again (5120 at 56: 29.5 against 26.4).
+//   - more, or wide: warps of 32 weight rows, whose two tiles share every activation operand and scale read from shared memory -
 //     its bandwidth is the bound at one tile per warp (head at 48 rows: 379 us against 418) - on CTA tiles of 64 x 64, 64 x 48
-//     or 128 x 24, whichever leaves the least idle in the last round of CTAs per SM.
+//     or 128 x 24, whichever leaves the least idle in the last round of CTAs per SM (7168 at 220 rows: 86.0 against 73.4); but
+//     where that is more than one round of the smallest tile and tcgen05's row blocks of 32 are one wave, these (5120 x 17408 at 72 rows
+//     87.8 against 92.5).  A last row block of at most eight rows costs little: it may lie a seventh over the wave.
 int launch_g32_any(const int8_t* a, const int8_t* w, const w8a8::SwapArgs& p, cudaStream_t st) {
     const int M = p.M, N = p.N;
-    const long sms = sm_count();
+    const long sms = sm_count(), tiles = (N + 127) / 128;
     const bool wide = N >= 16 * 8 * sms;
-    if (M > 16 && (long)((N + 127) / 128) * ((M + 15) / 16) <= sms && w8a8::G32::stages_for(p.K) >= 3)
-        return launch_g32(a, w, p, st);
-    if (M <= 8) return wide ? launch_g32_mma<1, 1, 2, 1, 2, 4>(a, w, p, st) : launch_g32_mma<1, 1, 1, 1, 4, 3>(a, w, p, st);
+    const bool can16 = w8a8::G32<16>::stages_for(p.K, 16) >= 3, can32 = w8a8::G32<32>::stages_for(p.K, 32) >= 3;
     if (M <= 16) {
+        if (!wide && tiles * 4 > sms * 3 && tiles <= sms && can16) return launch_g32<16>(a, w, p, st);
+        if (M <= 8) return wide ? launch_g32_mma<1, 1, 2, 1, 2, 4>(a, w, p, st) : launch_g32_mma<1, 1, 1, 1, 4, 3>(a, w, p, st);
         if (!wide) return launch_g32_mma<1, 1, 1, 2, 4, 3>(a, w, p, st);
         return N >= 64 * 8 * sms ? launch_g32_mma<2, 2, 2, 1, 2, 3>(a, w, p, st) : launch_g32_mma<2, 2, 4, 1, 1, 3>(a, w, p, st);
     }
-    if (M <= 64 && !wide) return launch_g32_mma<2, 1, 2, 2, 2, 4>(a, w, p, st);
+    if (tiles * ((M + 15) / 16) <= sms && can16) return launch_g32<16>(a, w, p, st);
+    if (M <= 64 && !wide) {
+        if ((M <= 32 || tiles * 3 > sms) && can32) return launch_g32<32>(a, w, p, st);
+        return launch_g32_mma<2, 1, 2, 2, 2, 4>(a, w, p, st);
+    }
     if (M <= 32) return launch_g32_mma<4, 2, 4, 1, 1, 3>(a, w, p, st);
     if (M <= 48) return launch_g32_mma<6, 2, 4, 1, 1, 3>(a, w, p, st);
     // rounds of CTAs per SM x the tile's 16 x 8 units x its measured time per unit
@@ -511,8 +520,11 @@ int launch_g32_any(const int8_t* a, const int8_t* w, const w8a8::SwapArgs& p, cu
         return ((long)((N + rows - 1) / rows) * ((M + mc - 1) / mc) + sms - 1) / sms * (rows / 16) * (mc / 8) * time;
     };
     const long c64 = cost(64, 64, 68), c48 = cost(64, 48, 68), c24 = cost(128, 24, 72);
-    if (c64 <= c48 && c64 <= c24) return launch_g32_mma<4, 2, 2, 2, 1, 4>(a, w, p, st);
-    return c48 <= c24 ? launch_g32_mma<3, 2, 2, 2, 1, 4>(a, w, p, st) : launch_g32_mma<3, 2, 4, 1, 1, 3>(a, w, p, st);
+    const long best = c64 < c48 ? (c64 < c24 ? c64 : c24) : (c48 < c24 ? c48 : c24);
+    if (best > 25 * 68 && tiles * ((M + 31) / 32) <= sms + (M % 32 && M % 32 <= 8 ? sms / 7 : 0) && can32)
+        return launch_g32<32>(a, w, p, st);
+    if (best == c64) return launch_g32_mma<4, 2, 2, 2, 1, 4>(a, w, p, st);
+    return best == c48 ? launch_g32_mma<3, 2, 2, 2, 1, 4>(a, w, p, st) : launch_g32_mma<3, 2, 4, 1, 1, 3>(a, w, p, st);
 }
 
 // Can those kernels take the call?  One K slice and a direct store.  PRISM_B200_G32=0 keeps the older kernel (comparisons).

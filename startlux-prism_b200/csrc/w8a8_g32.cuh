@@ -14,23 +14,24 @@
 //     of the fp32 pipe per 512 bytes of K and 8 rows a warp; it reads the activation scales, loaded once into shared
 //     memory, and never waits on a pipeline stage: the stages go back to the producer when their MMAs have completed.
 // Roles: warp 0 = TMA producer (one thread), warps 1 and 2 = MMA issuers (one thread each; warp 1 owns the tensor
-// memory), warps 3..10 = epilogue: two warps per lane quarter, each with 8 of the CTA's 16 activation rows.
-// Row blocks of 16 in grid.z, for the row counts whose blocks all fit one wave of CTAs; everything else runs on
-// w8a8_g32_mma.cuh.
+// memory), warps 3..10 = epilogue: two warps per lane quarter, each with RW = NB / 2 of the CTA's activation rows.
+// NB = 16 or 32: row blocks of that many activation rows in grid.z, for the row counts whose blocks all fit one wave of CTAs
+// (each block re-reads the weights from L2); everything else runs on w8a8_g32_mma.cuh.
 #pragma once
 #include "w8a8_gemm.cuh"
 
 namespace w8a8 {
 
+template <int NB_>
 struct G32 {
-    static constexpr int NB = 16;                         // MMA N: activation rows per CTA (zero-filled past M)
+    static constexpr int NB = NB_;                        // MMA N: activation rows per CTA (zero-filled past M): 16 or 32
     static constexpr int KS = 256;                        // bytes of K per stage
     static constexpr int W_BYTES = BM * KS;               // 32 KB: [2][128 rows][128 bytes], 128-byte swizzle
     static constexpr int X_BYTES = NB * KS;               // [2][NB rows][128 bytes]
     static constexpr int STAGE_BYTES = W_BYTES + X_BYTES;
     static constexpr int SLOT_COLS = 256;                 // an accumulator slot: 16 columns per group and row ...
-    static constexpr int SLOT_QUADS = SLOT_COLS / (4 * NB);   // ... = 4 quads (a quad = 4 groups = 128 bytes of K)
-    static constexpr int SLOT_STAGES = SLOT_QUADS / 2;    // stages per slot: 2
+    static constexpr int SLOT_QUADS = SLOT_COLS / (4 * NB);   // ... = 4 quads of 16 rows, 2 quads of 32 (a quad = 4 groups = 128 bytes of K)
+    static constexpr int SLOT_STAGES = SLOT_QUADS / 2;    // stages per slot: 2 or 1
     static constexpr int RING = 2;                        // 512 columns: one CTA per SM
     static constexpr int TMEM_COLS = 512;
     static constexpr int EPI_WARPS = 8;
@@ -40,12 +41,12 @@ struct G32 {
     static constexpr int MAX_STAGES = 5;
     // activation scales in shared memory: [rows][quads rounded up to a multiple of four] float4
     __host__ __device__ static constexpr int padded_quads(int K) { return (K / 128 + 3) / 4 * 4; }
-    __host__ __device__ static constexpr int sa_bytes(int K) { return NB * padded_quads(K) * 16; }
-    static constexpr int smem_bytes(int K, int stages) {
-        return 1024 + stages * STAGE_BYTES + sa_bytes(K) + (int)sizeof(Aux);
+    __host__ __device__ static constexpr int sa_bytes(int K, int rows) { return rows * padded_quads(K) * 16; }
+    static constexpr int smem_bytes(int K, int rows, int stages) {
+        return 1024 + stages * STAGE_BYTES + sa_bytes(K, rows) + (int)sizeof(Aux);
     }
-    static constexpr int stages_for(int K) {
-        const int room = 232448 - 1024 - (int)sizeof(Aux) - sa_bytes(K);
+    static constexpr int stages_for(int K, int rows) {
+        const int room = 232448 - 1024 - (int)sizeof(Aux) - sa_bytes(K, rows);
         return room / STAGE_BYTES > MAX_STAGES ? MAX_STAGES : room / STAGE_BYTES;
     }
 };
@@ -134,20 +135,21 @@ __device__ __forceinline__ void add_quad(f32x2* acc, const uint32_t (&r)[4][RW],
 }
 
 // tm_w: weights [N, K] as {128, N, K / 128} with box {128, 128, 2}; tm_x: activations [M, K] the same way with box
-// {128, 16, 2}.  p: a_s [M, K / 32], w_s [N, K / 32], out, ldo, n_rows, M, N, K (a multiple of 128), epi (bf16, fp32 add
-// or fp32), pdl, stages.  Grid (N / 128 tiles, 1, row blocks of 16).
-__global__ void __launch_bounds__(G32::THREADS, 1)
+// {128, NB, 2}.  p: a_s [M, K / 32], w_s [N, K / 32], out, ldo, n_rows, M, N, K (a multiple of 128), epi (bf16, fp32 add
+// or fp32), pdl, stages.  Grid (N / 128 tiles, 1, row blocks of 2 * RW).
+template <int NB, int RW>
+__global__ void __launch_bounds__(G32<NB>::THREADS, 1)
 w8a8_g32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const SwapArgs p) {
-    using C = G32;
-    constexpr int NB = C::NB, RW = 8;                          // activation rows of the CTA, of a warp
-    constexpr int RCTA = NB, RC = RW;                          // ... and rows per tensor-memory load
+    using C = G32<NB>;
+    constexpr int RCTA = 2 * RW;                               // activation rows this CTA owns (<= NB)
+    constexpr int RC = RW < 8 ? RW : 8;                        // rows per tensor-memory load
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = align1024(smem_raw);
     const int NST = p.stages;
     const int KC = p.K / BK;                                   // quads = 128-byte chunks of K
     const int QP = C::padded_quads(p.K);
     float4* sa = (float4*)(smem + NST * C::STAGE_BYTES);       // float2 [RCTA / 2 row pairs][QP quads][4 groups]
-    Aux* aux = (Aux*)((uint8_t*)sa + C::sa_bytes(p.K));
+    Aux* aux = (Aux*)((uint8_t*)sa + C::sa_bytes(p.K, RCTA));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     int live = *p.n_rows;

@@ -340,7 +340,8 @@ def test_l2_prefetch(dev):
 
 
 @pytest.mark.parametrize("M,N,K,live", [(3, 20, 128, 3), (9, 33, 384, 8), (30, 1000, 640, 30), (50, 200, 256, 49),
-                                        (8, 18945, 256, 7), (16, 18960, 128, 16), (16, 75800, 128, 15), (17, 19000, 128, 17),
+                                        (8, 18945, 256, 7), (16, 18960, 128, 16), (12, 17408, 128, 12), (40, 7168, 128, 40),
+                                        (72, 7168, 128, 71), (56, 5120, 384, 56), (16, 75800, 128, 15), (17, 19000, 128, 17),
                                         (33, 19000, 128, 33), (64, 19000, 128, 60), (65, 130, 384, 65), (500, 7168, 256, 499),
                                         (256, 34816, 128, 256)])
 def test_groups_of_32_every_tile(dev, M, N, K, live):
