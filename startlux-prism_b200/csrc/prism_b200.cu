@@ -633,27 +633,27 @@ int launch_w4a8_few(const w4a8::GemvArgs& p, cudaStream_t st) {
     return p.M <= 16 ? launch_w4a8_mma<KIND, 2, 2, 2, 4, 2>(p, st) : launch_w4a8_mma<KIND, 4, 1, 4, 2, 2>(p, st);
 }
 
-// One or two activation rows against Q6_K: integer dot products on the CUDA cores (w4a8_gemv.cuh).
+// One activation row (two for Q6_K): integer dot products on the CUDA cores (w4a8_gemv.cuh).
 template <int MR>
-int launch_w4a8_gemv(const w4a8::GemvArgs& p, cudaStream_t st) {
+int launch_w4a8_gemv(int kind, const w4a8::GemvArgs& p, cudaStream_t st) {
     constexpr int R = w4a8::GEMV_R;
     const int grid = (p.N + 4 * R - 1) / (4 * R);                  // eight weight rows per CTA
-    auto split_k = w4a8::w4a8_gemv_q6k_kernel<MR, R, true>;
-    auto whole_k = w4a8::w4a8_gemv_q6k_kernel<MR, R, false>;
+    auto split_k = kind == 0 ? w4a8::w4a8_gemv_q4k_kernel<MR, R, true> : w4a8::w4a8_gemv_q6k_kernel<MR, R, true>;
+    auto whole_k = kind == 0 ? w4a8::w4a8_gemv_q4k_kernel<MR, R, false> : w4a8::w4a8_gemv_q6k_kernel<MR, R, false>;
     // few rows: two to four warps per CTA share the rows' super-blocks (exact: the chain runs in order afterwards);
     // the most warps with which the whole grid is resident at once (a second, short wave would double the time)
     const size_t smem = (size_t)(p.K >> 8) * 4 * R * MR * sizeof(float);
     if (grid < 8 * sm_count() && smem <= 48 * 1024) {
-        static int resident_dev[kMaxDevices][5] = {};              // [device][warps] CTAs per SM, 0 = not asked yet
-        int (&resident)[5] = resident_dev[current_device()];
+        static int resident_dev[kMaxDevices][2][5] = {};           // [device][kind][warps] CTAs per SM, 0 = not asked yet
+        int (&resident)[2][5] = resident_dev[current_device()];
         int kw = 2;
         for (int k = 4; k >= 2; --k) {
-            if (!resident[k]) {
+            if (!resident[kind][k]) {
                 int nb = 0;
                 PB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, split_k, 32 * k, 16 * 1024));
-                resident[k] = nb > 0 ? nb : 1;
+                resident[kind][k] = nb > 0 ? nb : 1;
             }
-            if ((long)grid <= (long)resident[k] * sm_count()) {
+            if ((long)grid <= (long)resident[kind][k] * sm_count()) {
                 kw = k;
                 break;
             }
@@ -730,7 +730,7 @@ bool w8a8_no_gemv() {
     return v == 1;
 }
 
-// PRISM_B200_W4A8_NO_GEMV=1 keeps the tensor-core kernels for one and two Q6_K rows (comparison runs).
+// PRISM_B200_W4A8_NO_GEMV=1 keeps the tensor-core kernels for one and two rows (comparison runs).
 bool w4a8_no_gemv() {
     static int v = -1;
     if (v < 0) {
@@ -1490,14 +1490,15 @@ int pb_w4a8_gemm(const int8_t* xq, const float* a, const int8_t* xs, int Ma, int
         if (workspace_bytes < pb_w4a8_workspace_bytes(M, N, K) || n_counters < pb_w4a8_counters(M, N)) return PB_TOO_LARGE;
     }
     // Up to 32 rows, or 64 against so few weight rows that the many-rows kernel's 64-column tiles leave most SMs idle (at
-    // 50 rows 12.9 against 29 us on 1024 rows of Q6_K, but 25 against 23 on 5120 of Q4_K).  One or two Q6_K rows stay on
-    // the CUDA cores (5120 x 17408: 20.5 / 22.4 us against 23.7; from four rows on 24.0 against 30.5).
+    // 50 rows 12.9 against 29 us on 1024 rows of Q6_K, but 25 against 23 on 5120 of Q4_K).  One row stays on
+    // the CUDA cores (a whole layer 77 us against 81), and two against many Q6_K rows (5120 x 17408: 22.4 us against 23.7; from four
+    // rows on 24.0 against 30.5).
     if ((M <= 32 || (M <= 64 && N <= 16 * sm_count())) && !w4a8_tile_only()) {
         const w4a8::GemvArgs g{xq, a, xs, (const uint8_t*)wq, (const uint8_t*)wsc, (const uint8_t*)wmn, wd, wdm, out, ldo, n_rows,
                                M, N, K, Ma, epi};
+        if (M == 1 && !w4a8_no_gemv()) return launch_w4a8_gemv<1>(kind, g, st);
         if (kind == 0) return launch_w4a8_few<w4a8::KIND_Q4K>(g, st);
-        if (M <= 2 && N > 16 * sm_count() && !w4a8_no_gemv())
-            return M == 1 ? launch_w4a8_gemv<1>(g, st) : launch_w4a8_gemv<2>(g, st);
+        if (M == 2 && N > 16 * sm_count() && !w4a8_no_gemv()) return launch_w4a8_gemv<2>(kind, g, st);
         return launch_w4a8_few<w4a8::KIND_Q6K>(g, st);
     }
     if (kind == 0)

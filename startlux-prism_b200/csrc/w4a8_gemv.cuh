@@ -1,20 +1,28 @@
-// W4A8 for one or two activation rows against Q6_K: no tensor core - at these row counts it would be a few per cent used -
-// but integer dot products on the CUDA cores, straight from the packed weights in global memory.  Same arithmetic as the
-// other W4A8 kernels (kernels/w4a8.py:14-24): exact integers inside a 256-input super-block, then per super-block, in
-// order, y = fma(a, d * float(acc), y).  (Q4_K at these row counts runs on mma.sync: w4a8_mma.cuh.)
+// W4A8 for one activation row (two against Q6_K matrices of many rows; w4a8_mma.cuh takes over from there: a layer at two rows
+// 90 -> 81 us, but 77 -> 81 at one): no tensor core - at these row counts the MMA
+// would be 3 % used and the hand-offs between its stages are what the time goes to - but integer dot products on the
+// CUDA cores, straight from the packed weights in global memory.  Same arithmetic as the other W4A8 kernels
+// (kernels/w4a8.py:14-24): exact integers inside a 256-input super-block, then per super-block, in order,
+//   Q4_K  t = d * float(acc); t = fma(-dmin, float(mins), t); y = fma(a, t, y)
+//   Q6_K  y = fma(a, d * float(acc), y)
 //
 // Eight lanes share a weight row's super-block, 32 inputs each, and take R = 2 rows at a time, so a warp covers eight
-// rows and a warp instruction reads whole 128-byte lines: a lane's 32 int8 values are two 16-input sub-blocks with an int8
-// scale each: eight dp4a, two multiplies.
+// rows and a warp instruction reads whole 128-byte lines:
+//   Q4_K  a lane's share of a row is one 32-input sub-block = 16 packed bytes (byte t = q[t] | q[t + 16] << 4): four
+//         words, split into low and high nibbles, eight dp4a against the activations' 32 bytes (held in registers for
+//         both rows), times the sub-block's 6-bit scale;
+//   Q6_K  32 int8 values = two 16-input sub-blocks with an int8 scale each: eight dp4a, two multiplies.
 // The R x M partial sums are then added over the eight lanes by a halving exchange (each step a lane keeps half of its
 // values and sends the other half: R x M - 1 shuffles instead of 3 R x M), which leaves every (row, activation row)
-// pair's exact integer in one lane; that lane owns the pair's fp32 chain.
-// Everything that comes from HBM once - the weights, their sub-block scales and the super-block's d -
+// pair's exact integer in one lane; that lane owns the pair's fp32 chain.  Q4_K's mins term needs no exchange: the
+// owner forms it from the row's eight 6-bit mins and the activation row's eight group sums with four dp4a (the sums
+// are stored as S & 63 and S >> 6, both inside int8).
+// Everything that comes from HBM once - the weights, their sub-block scales and mins, the super-block's d and dmin -
 // is loaded for PD super-blocks at a time into registers (about 150 bytes per lane and super-block), all requests
 // issued before the first use; the PD super-blocks are then worked through while other warps' requests are in flight.
 // (A rolling register prefetch, one super-block consumed and one requested per step, measured at a third of the HBM
-// rate: a wait for the oldest request also waits for the younger ones that share its scoreboard.)  Activations and
-// their scales are small and stay in L1.  A CTA is one warp: eight rows, so that even a 5120-row projection
+// rate: a wait for the oldest request also waits for the younger ones that share its scoreboard.)  Activations, their
+// group sums and scales are small and stay in L1.  A CTA is one warp: eight rows, so that even a 5120-row projection
 // spreads evenly over the SMs; for matrices of few rows a CTA is two to four warps on the same eight rows, each
 // taking every KW-th super-block: its terms of the chain meet in shared memory and are added in order by one thread
 // per output, so the bits do not depend on the split.
@@ -123,6 +131,105 @@ __device__ __forceinline__ void gemv_chain(const GemvArgs& p, const float* terms
     float y = 0.0f;
     for (int b = 0; b < NSB; ++b) y = __fmaf_rn(__ldg(p.a + (long)b * p.Ma + mm), terms[b * (4 * NV) + t], y);
     gemv_store(p, y, (long)blockIdx.x * 4 * R + t / MR, m, live, true);
+}
+
+template <int MR, int R, bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? 128 : 32)
+w4a8_gemv_q4k_kernel(const GemvArgs p) {
+    constexpr int NV = R * MR, PD = GEMV_PD, NF = NV >= 8 ? NV / 8 : 1;   // NF: (row, activation row) pairs per lane
+    extern __shared__ float gemv_terms[];                          // SPLIT: [K / 256][4 * R * MR] chain terms
+    const int KW = SPLIT ? (int)(blockDim.x >> 5) : 1;             // warps sharing the CTA's rows
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = lane & 7;                                        // sub-block of the super-block
+    const long n0 = ((long)blockIdx.x * 4 + (lane >> 3)) * R;
+    int live = *p.n_rows;
+    live = live < p.M ? live : p.M;
+    if (live <= 0) return;
+    const int NSB = p.K >> 8;
+    // the (row, activation row) pairs whose fp32 chains this lane owns: NF consecutive activation rows of one row
+    const int mine = reduce8_index<NV>(lane), r_o = mine / MR, m_o = mine % MR;
+    const long row_o = n0 + r_o < p.N ? n0 + r_o : p.N - 1;        // rows past N read the last row and store nothing
+    const uint8_t* wrow[R];
+    const uint8_t* scrow[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const long nn = n0 + r < p.N ? n0 + r : p.N - 1;
+        wrow[r] = p.wq + nn * (p.K >> 1) + g * 16;
+        scrow[r] = p.sc + nn * 8 + g;
+    }
+    const long sb_stride = (long)p.N * 8;
+    uint4 ring[PD][R];
+    int sc[PD][R];
+    uint2 mn[PD];
+    float dv[PD], dmv[PD];
+    float y[NF];
+#pragma unroll
+    for (int i = 0; i < NF; ++i) y[i] = 0.0f;
+    for (int b0 = warp; b0 < NSB; b0 += PD * KW) {
+#pragma unroll
+        for (int j = 0; j < PD; ++j)
+            if (b0 + j * KW < NSB) {
+                const long b = b0 + j * KW;
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    ring[j][r] = ldg_stream(wrow[r] + b * 128);
+                    sc[j][r] = scrow[r][b * sb_stride];
+                }
+                mn[j] = __ldg((const uint2*)(p.mn + (b * p.N + row_o) * 8));
+                dv[j] = __ldg(p.d + b * p.N + row_o);
+                dmv[j] = __ldg(p.dm + b * p.N + row_o);
+            }
+#pragma unroll
+        for (int j = 0; j < PD; ++j) {
+            const int b = b0 + j * KW;
+            if (b < NSB) {
+                uint4 w[R];
+                int scb[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    w[r] = ring[j][r];
+                    scb[r] = sc[j][r];
+                }
+                const uint2 mnb = mn[j];
+                const float dvb = dv[j], ndm = -dmv[j];
+                uint4 x0[MR], x1[MR];
+#pragma unroll
+                for (int m = 0; m < MR; ++m) {
+                    const int mm = m < p.M ? m : p.M - 1;
+                    const uint4* xp = (const uint4*)(p.xq + (long)mm * p.K + b * 256 + g * 32);
+                    x0[m] = __ldg(xp);                             // inputs 0..15 and 16..31 of the sub-block
+                    x1[m] = __ldg(xp + 1);
+                }
+                int v[NV];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const uint4 lo = {w[r].x & 0x0F0F0F0Fu, w[r].y & 0x0F0F0F0Fu, w[r].z & 0x0F0F0F0Fu, w[r].w & 0x0F0F0F0Fu};
+                    const uint4 hi = {(w[r].x >> 4) & 0x0F0F0F0Fu, (w[r].y >> 4) & 0x0F0F0F0Fu, (w[r].z >> 4) & 0x0F0F0F0Fu,
+                                      (w[r].w >> 4) & 0x0F0F0F0Fu};
+#pragma unroll
+                    for (int m = 0; m < MR; ++m) v[r * MR + m] = scb[r] * dot32(lo, hi, x0[m], x1[m]);
+                }
+                reduce8<NV>(v, lane);
+#pragma unroll
+                for (int i = 0; i < NF; ++i) {                     // this lane's pairs: the same row, consecutive m
+                    const int mi = m_o + i < p.M ? m_o + i : p.M - 1;
+                    const uint4 s = __ldg((const uint4*)(p.xs + ((long)b * p.Ma + mi) * 16));
+                    const int mins = __dp4a((int)mnb.x, (int)s.x, __dp4a((int)mnb.y, (int)s.y, 0)) +
+                                     64 * __dp4a((int)mnb.x, (int)s.z, __dp4a((int)mnb.y, (int)s.w, 0));
+                    float t = __fmul_rn(dvb, __int2float_rn(v[i]));
+                    t = __fmaf_rn(ndm, __int2float_rn(mins), t);
+                    if (!SPLIT) y[i] = __fmaf_rn(__ldg(p.a + (long)b * p.Ma + mi), t, y[i]);
+                    else if (reduce8_owner<NV>(lane)) gemv_terms[b * (4 * NV) + ((lane >> 3) * R + r_o) * MR + m_o + i] = t;
+                }
+            }
+        }
+    }
+    if (!SPLIT) {
+#pragma unroll
+        for (int i = 0; i < NF; ++i) gemv_store(p, y[i], n0 + r_o, m_o + i, live, reduce8_owner<NV>(lane));
+    } else {
+        gemv_chain<MR, R>(p, gemv_terms, NSB, live);
+    }
 }
 
 template <int MR, int R, bool SPLIT>
