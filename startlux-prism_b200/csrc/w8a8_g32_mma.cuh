@@ -65,11 +65,11 @@ w8a8_g32_mma_kernel(const int8_t* __restrict__ a, const int8_t* __restrict__ w, 
         for (int i = 0; i < C::ROWS / STEP; ++i)
             if (r0 + i * STEP < nrows)
                 cp_async16(sb + (d0 ^ (((i * STEP) & 7) << 4)) + i * STEP * 128, wsrc + (long)i * STEP * p.K + kc * 128);
+    };
+    auto load_x = [&](int kc, uint32_t sb) {                      // activations and both operands' scales
 #pragma unroll
         for (int i = 0; i < (C::ROWS + T - 1) / T; ++i)
             if (tid + i * T < nrows) cp_async16(sb + C::OFF_SW + (tid + i * T) * 16, swsrc + (long)i * T * G + kc * 4);
-    };
-    auto load_x = [&](int kc, uint32_t sb) {
 #pragma unroll
         for (int i = 0; i < (C::MC + STEP - 1) / STEP; ++i) {
             const int m = r0 + i * STEP;
@@ -92,7 +92,8 @@ w8a8_g32_mma_kernel(const int8_t* __restrict__ a, const int8_t* __restrict__ w, 
     const f32x2 unbias = pack2(-12582912.0f, -12582912.0f);
     const int R = (KC + KQ - 1) / KQ;
 
-    // a programmatic dependent requests its first weights before it waits for the producer of the activations
+    // a programmatic dependent requests its first int8 weights, and nothing else, before it waits for the kernel before it:
+    // that one may write the activations and the scales of either operand
 #pragma unroll
     for (int s = 0; s < ST - 1; ++s)
 #pragma unroll

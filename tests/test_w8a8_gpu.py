@@ -363,3 +363,31 @@ def test_groups_of_32_every_tile(dev, M, N, K, live):
         w8a8.gemm(*dargs, f, n_rows(live, dev), 32, epi=w8a8.EPI_F32)
         ref = oracle.w8a8_gemm(*args, 4, live)
         assert np.array_equal(f.cpu().numpy()[:live], ref[:live]) and bool((f[live:] == 7.0).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(8, 640, 1024), (12, 17408, 256), (40, 19000, 256), (56, 5120, 512)])
+def test_dependent_reads_weight_scales_after_the_wait(dev, M, N, K):
+    """pdl=True and per-32 groups: the kernel before (a fold, which lets its dependents start at once and then takes its
+    time over 400 slots) writes the weights' scales; only the int8 weights may be read before it has ended - on the warp-level
+    tiles and on the tcgen05 kernel (12 rows) alike."""
+    from prism_b200 import _lib
+    G, S = K // 32, 400
+    a, w, sa, _ = rand_w8a8(M, N, K, seed=N + M, groups=G)
+    g = torch.Generator().manual_seed(N)
+    part = torch.randint(1, 100, (N, G), generator=g, dtype=torch.int32)
+    rs, cs = torch.rand(N, generator=g) * 1e-3, torch.rand(G, generator=g) * 1e-2
+    sw = oracle.fold(np.zeros((N, G), np.float32), (part.numpy().astype(np.int64) * S).astype(np.int32)[None], rs.numpy(), cs.numpy())
+    ref = oracle.w8a8_gemm(a.numpy(), sa.numpy(), w.numpy(), sw, 32, 0)
+    ad, wd, sad = a.to(dev), w.to(dev), sa.to(dev)
+    slots, pend = part.to(dev).expand(S, N, G).contiguous(), w8a8.Deferred(S, rs.to(dev), cs.to(dev))
+    swd, out = torch.empty(N, G, device=dev), torch.empty(M, N, dtype=torch.bfloat16, device=dev)
+    nr, nw = n_rows(M, dev), n_rows(N, dev)
+    before = _lib.lib().pb_set_pdl(1)
+    try:
+        for _ in range(5):
+            swd.zero_()
+            quant.fold(swd, slots, pend, nw, N)
+            w8a8.gemm(ad, sad, wd, swd, out, nr, 32, pdl=True)
+            assert same(swd, sw) and same(out, bf16_from_bits(ref)), first_diff(np_bits(out), ref)
+    finally:
+        _lib.lib().pb_set_pdl(before)
