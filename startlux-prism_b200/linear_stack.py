@@ -84,8 +84,11 @@ class LinearStack:
         # 0.402 at 64, as a replayed graph.  One row too, on the tensor-core kernel then: 0.318 ms with the CUDA-core GEMM's
         # plain launches, 0.297 as a chain (0.42 with that GEMM as a dependent).  PRISM_B200_PDL=0 keeps plain launches.
         self.pdl = n == 1 and M <= w8a8.FEW_ROWS and os.environ.get("PRISM_B200_PDL", "1") != "0"
-        if self.pdl and self.h.is_cuda:
-            w8a8._workspace_if_ready(self.h.device)   # the tensor-core kernel's split-K array: a pass can be captured unrun
+        # a few-row pass adds its K splits in memory of its own (2 to 4 MB at the 27B shapes): the passes of two stacks may
+        # overlap on two streams, and a pass can be captured unrun
+        self.scratch = None
+        if M <= w8a8.FEW_ROWS:
+            self.scratch = w8a8.Scratch(M, [(*lw[k][0].shape, k in ("o", "down")) for lw in layers for k in lw], device, self.pdl)
         # several ranks and many rows: the residual stream stays split by rows between the projections (each rank
         # folds, normalises and quantizes M / n rows), a row-parallel projection's int32 sums are reduce-scattered and
         # the int8 rows of the next projection's input all-gathered: 5/8 of an all-reduce's bytes, and 1 / n of the
@@ -166,12 +169,12 @@ class LinearStack:
         pend = None
         for lw in self.layers:
             quant.fold_rows_q8(self.h, self.slots, pend, self.xq, self.xs, nr, M)
-            w8a8.gemm(self.xq, self.xs, *lw["qkv"], self.qkv, nr, self.hidden, pdl=self.pdl)
+            w8a8.gemm(self.xq, self.xs, *lw["qkv"], self.qkv, nr, self.hidden, pdl=self.pdl, scratch=self.scratch)
             tp.quantize_rows(g if self.n > 1 else None, quant.rows_q8, M, self.amax, self.qkv[:, :self.ql], None,
                              self.aq, self.as_, nr, M)
             pend = self._out(self.aq, self.as_, lw["o"])
             quant.fold_rows_q8(self.h, self.slots, pend, self.xq, self.xs, nr, M)
-            w8a8.gemm(self.xq, self.xs, *lw["gate_up"], self.gu, nr, self.hidden, pdl=self.pdl)
+            w8a8.gemm(self.xq, self.xs, *lw["gate_up"], self.gu, nr, self.hidden, pdl=self.pdl, scratch=self.scratch)
             tp.quantize_rows(g if self.n > 1 else None, quant.swiglu_q8, M, self.amax, self.gu, None, self.dq,
                              self.ds, nr, M)
             pend = self._out(self.dq, self.ds, lw["down"])
@@ -189,7 +192,8 @@ class LinearStack:
         w, w_s = wt
         if self.n > 1:
             return tp.out_proj(self.g, a, a_s, w, w_s, self.parts, self.M, self.n_rows, pdl=self.pdl)
-        return w8a8.gemm(a, a_s, w, w_s, self.h, self.n_rows, a.shape[1], epi=1, slots=self.slots, pdl=self.pdl)
+        return w8a8.gemm(a, a_s, w, w_s, self.h, self.n_rows, a.shape[1], epi=1, slots=self.slots, pdl=self.pdl,
+                         scratch=self.scratch)
 
     def _pass_by_rows(self, gather=True):
         """Several ranks, many rows.  Between a row-parallel projection and the next column-parallel one every rank

@@ -14,6 +14,7 @@ Kernel choice (this module's table replaces the reference's per-GPU JSON tables)
 128 x 256 tile kernel; up to 64 rows -> the operand-swapped split-K kernel, the splits' int32 sums either deferred to
 the caller's `slots` (epi 1) or added inside the kernel through a workspace.
 """
+import weakref
 from typing import NamedTuple
 
 import torch
@@ -44,9 +45,9 @@ class Deferred(NamedTuple):
 
 def _workspace(device):
     """(workspace bytes tensor, zeroed int32 counters) of a device; allocated once, outside any graph capture.  One
-    array per device, shared by the W8A8, W4A8 and MXFP4 split-K kernels on whatever stream calls them: two products
-    that split K and overlap on the GPU (different streams) race on it - keep split-K products of one device on one
-    stream, or give the second stream its own arrays through the C entry points."""
+    array per device, shared by the W8A8 and MXFP4 split-K kernels on whatever stream calls them: two products that
+    split K and overlap on the GPU (different streams) race on it - keep split-K products of one device on one stream,
+    or give the second stream its own (gemm's `scratch`, or the C entry points' arguments)."""
     key = torch.device(device).index or 0
     if key not in _WORKSPACE:
         if torch.cuda.is_current_stream_capturing():
@@ -65,12 +66,37 @@ def _workspace_if_ready(device):
     return _workspace(device)
 
 
+_SCRATCH = weakref.WeakSet()     # every live Scratch: reset_workspace zeroes their counters too
+
+
+class Scratch:
+    """Split-K partial sums and arrival counters of one owner, for products that may run beside other streams' products:
+    gemm(..., scratch=) uses them in place of the device's shared array.  products: the (N, K, residual) of the few-row
+    (gk == K) products it will serve at M rows, one after the other on one stream; pdl as the products will be called."""
+
+    def __init__(self, M, products, device, pdl=False):
+        L = _lib.lib()
+        need = count = 0
+        for N, K, residual in products:
+            split = effective_split(K, _few_split(M, N, K, residual, pdl)[0])
+            if split > 1:
+                need = max(need, L.pb_w8a8_workspace_bytes(M, N, split))
+                count = max(count, L.pb_w8a8_counters(M, N))
+        self.ws = torch.empty(need, dtype=torch.uint8, device=device)
+        self.counters = torch.zeros(count, dtype=torch.int32, device=device)
+        _SCRATCH.add(self)
+
+
 def reset_workspace(device=None):
     """Zero the split-K arrival counters (after a kernel reported PB_DEVICE_TIMEOUT: a CTA that gave up a wait did not
     count itself in, so its tile's counter is left non-zero)."""
+    want = None if device is None else torch.device(device).index or 0
     for key, (_, counters) in _WORKSPACE.items():
-        if device is None or key == (torch.device(device).index or 0):
+        if want is None or key == want:
             counters.zero_()
+    for x in list(_SCRATCH):
+        if want is None or (x.counters.device.index or 0) == want:
+            x.counters.zero_()
 
 
 GEMV_ROWS = 1        # gk == K: this many rows against few weight rows run on the CUDA cores (PB_W8A8_GEMV_ROWS)
@@ -94,7 +120,7 @@ def pick_split(M, N, K, limit=MAX_SPLIT):
 _TABLE = None
 
 
-def _choice(M, N, K, residual, pdl=False):
+def _choice(M, N, K, residual, chained=False):
     """The measured choice for this projection shape at the nearest measured row count (tune.py's table), or None."""
     global _TABLE
     if _TABLE is None:
@@ -105,8 +131,8 @@ def _choice(M, N, K, residual, pdl=False):
         return None
     import math
     # the one-row entry was measured on the CUDA-core kernel: it says nothing about the tensor-core kernel, which runs at
-    # two rows up and for a programmatic dependent of one row
-    rows = [x for x in by_m if x > GEMV_ROWS] if M > GEMV_ROWS or pdl else list(by_m)
+    # two rows up and in a chain of programmatic dependents of one row
+    rows = [x for x in by_m if x > GEMV_ROWS] if M > GEMV_ROWS or chained else list(by_m)
     if not rows:
         return None
     m = min(rows, key=lambda x: abs(math.log(x) - math.log(max(M, 1))))
@@ -120,6 +146,12 @@ def effective_split(K, split):
     split = max(1, min(split, kb))
     per = -(-kb // split)
     return -(-kb // per)
+
+
+def _few_split(M, N, K, residual, chained):
+    """(K splits, may they be deferred to slots) of a few-row product: the table's choice or pick_split's."""
+    c = _choice(M, N, K, residual, chained)
+    return (c["split"], c["defer"]) if c else (pick_split(M, N, K), True)
 
 
 def _call(a, a_s, w, w_s, out, ldo, n_rows, gk, epi, split, slot_stride=0, ws=None, counters=None, pdl=False):
@@ -145,12 +177,14 @@ def _scales_ok(s, rows, groups, what):
         raise RuntimeError(f"w8a8.gemm: {what} must be contiguous fp32 with {rows} x {groups} elements")
 
 
-def gemm(a, a_s, w, w_s, out, n_rows, gk, epi=0, outs=None, cfg=None, slots=None, pdl=False):
+def gemm(a, a_s, w, w_s, out, n_rows, gk, epi=0, outs=None, cfg=None, slots=None, pdl=False, scratch=None):
     """a int8 [M, K], a_s fp32 [M, K/gk], w int8 [N, K], w_s fp32 [N, K/gk] -> out: bf16 [M, N] (epi 0) or added into
     fp32 [M, N] (epi 1); out may be a column slice of a wider buffer (its row stride is honoured).  Returns a Deferred
     when an epi 1 product split K into `slots` (int32 [S, rows, N]), else None.  cfg: None or the number of K splits.
     pdl: the few-rows kernel is launched as a programmatic dependent of the kernel before it on the stream: its
-    weights stream while that kernel (the producer of a and a_s) still runs; everything else waits for it."""
+    weights stream while that kernel (the producer of a and a_s) still runs; everything else waits for it.
+    scratch: a Scratch for K splits that are added inside the kernel, instead of the device's shared workspace; a
+    one-row dependent splits K there only if it has one."""
     M, K = a.shape
     N = w.shape[0]
     if epi == EPI_SWIGLU:
@@ -172,7 +206,7 @@ def gemm(a, a_s, w, w_s, out, n_rows, gk, epi=0, outs=None, cfg=None, slots=None
         split = effective_split(K, int(cfg)) if cfg is not None and M <= FEW_ROWS else 1
         ws = counters = None
         if split > 1:
-            ws, counters = _workspace(a.device)
+            ws, counters = (scratch.ws, scratch.counters) if scratch else _workspace(a.device)
         _call(a, a_s, w, w_s, out, out.stride(0), n_rows, gk, epi, split, 0, ws, counters, pdl=pdl)
         return None
     if cfg is None and not pdl and K % 256 == 0 and M <= GEMV_ROWS and (N + 7) // 8 < 8 * SM_COUNT:
@@ -182,10 +216,10 @@ def gemm(a, a_s, w, w_s, out, n_rows, gk, epi=0, outs=None, cfg=None, slots=None
     defer_ok = True
     if cfg is not None:
         split = int(cfg)
+    elif M <= FEW_ROWS:
+        split, defer_ok = _few_split(M, N, K, epi == EPI_ADD, pdl and scratch is not None)
     else:
-        c = _choice(M, N, K, epi == EPI_ADD, pdl) if M <= FEW_ROWS else None
-        split = c["split"] if c else pick_split(M, N, K)
-        defer_ok = c["defer"] if c else True
+        split = pick_split(M, N, K)
     split = effective_split(K, split)
     if split > 1 and M <= FEW_ROWS and epi == EPI_ADD and slots is not None and slots.shape[1] >= M and defer_ok:
         split = effective_split(K, min(split, slots.shape[0]))
@@ -195,7 +229,9 @@ def gemm(a, a_s, w, w_s, out, n_rows, gk, epi=0, outs=None, cfg=None, slots=None
             return Deferred(split, a_s, w_s)
     ws = counters = None
     if split > 1:
-        ws, counters = _workspace(a.device)
+        ws, counters = (scratch.ws, scratch.counters) if scratch else _workspace(a.device)
+        if scratch and _lib.lib().pb_w8a8_counters(M, N) > counters.numel():
+            split = 1
         while split > 1 and _lib.lib().pb_w8a8_workspace_bytes(M, N, split) > ws.numel():
             split -= 1
         if split == 1:

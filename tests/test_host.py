@@ -37,6 +37,67 @@ def test_operators_refuse_cpu_tensors(lib):
                   torch.tensor([4], dtype=torch.int32), 64)
 
 
+class _Recorder:
+    """The library with every launch replaced by a note of its arguments."""
+
+    def __init__(self, real):
+        self.real, self.gemms = real, []
+
+    def __getattr__(self, name):
+        if name.endswith(("_bytes", "_counters")) or name == "pb_set_pdl":
+            return getattr(self.real, name)
+
+        def launch(*args):
+            if name == "pb_w8a8_gemm":
+                self.gemms.append(args)
+            return 0
+        return launch
+
+
+@pytest.mark.parametrize("M", [1, 2, 16, 64])
+def test_few_row_stacks_share_no_workspace(lib, monkeypatch, M):
+    """Two stacks of the 27B shapes may have their passes in flight on two streams: a product that splits K inside the
+    kernel must be given partial sums and counters that belong to its own stack, with room for it."""
+    from prism_b200 import linear_stack as LS
+    rec = _Recorder(lib)
+    monkeypatch.setattr(_lib, "lib", lambda: rec)
+    monkeypatch.setattr(_lib, "need_cuda", lambda *t: None)
+    monkeypatch.setattr(_lib, "stream", lambda: 0)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(w8a8, "_WORKSPACE", {})
+
+    class Weights:                                  # shapes only: no memory is touched
+        def __init__(self, n, k):
+            self.shape, self.dtype = (n, k), torch.int8
+
+        def is_contiguous(self):
+            return True
+
+        def data_ptr(self):
+            return 4096
+    shapes = {"qkv": (7168, 5120), "o": (5120, 5120), "gate_up": (34816, 5120), "down": (5120, 17408)}
+    layers = [{name: (Weights(n, k), torch.ones(n)) for name, (n, k) in shapes.items()}]
+    used = []
+    for _ in range(2):
+        stack = LS.LinearStack(layers, M, torch.device("cpu"))
+        rec.gemms.clear()
+        stack(torch.zeros(M, 5120))
+        assert len(rec.gemms) == 4
+        ws = [(g[14], g[16]) for g in rec.gemms if g[14] is not None]
+        for g in rec.gemms:
+            m, n, epi, split = g[7], g[8], g[11], g[12]
+            if split > 1 and epi != w8a8.EPI_I32:
+                assert g[15] >= lib.pb_w8a8_workspace_bytes(m, n, split) and g[17] >= lib.pb_w8a8_counters(m, n)
+        used.append((stack, ws))
+    assert used[0][1], "q|k|v splits K inside the kernel at every few-row count"
+    assert not set(used[0][1]) & set(used[1][1]) and not w8a8._WORKSPACE
+    # what a kernel that gave up leaves behind is cleared there as well
+    scratch = used[0][0].scratch
+    scratch.counters.fill_(1)
+    w8a8.reset_workspace()
+    assert not scratch.counters.any()
+
+
 def test_argument_checks_without_gpu(lib):
     """Bad arguments are refused before any CUDA call."""
     assert lib.pb_w8a8_gemm(None, None, None, None, None, 0, None, 1, 1, 16, 16, 0, 1, 0, None, 0, None, 0, 0, None) == 1

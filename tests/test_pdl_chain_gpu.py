@@ -44,3 +44,37 @@ def test_chain_of_programmatic_dependents(M):
         assert torch.equal(out.view(torch.int32), want.view(torch.int32))
     code, where = _lib.device_status()
     assert code == 0, (code, hex(where))
+
+
+@pytest.mark.parametrize("M", [1, 16])
+def test_two_stacks_on_two_streams(M):
+    """Two users' decode passes side by side, eagerly and as two replayed graphs captured without an eager pass: each
+    stack splits K in memory of its own, so each gives the bits it gives alone."""
+    dev = torch.device("cuda:0")
+    g = torch.Generator().manual_seed(M)
+    stacks = [build(M, dev, True) for _ in range(2)]
+    inputs = [(torch.randn(M, HID, generator=g) * 0.5).to(dev) for _ in range(2)]
+    want = [build(M, dev, False)(h).clone() for h in inputs]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    graphs = []
+    torch.cuda.synchronize()
+    for stack, h, s in zip(stacks, inputs, streams):
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1], stream=s):
+            for _ in range(8):
+                stack(h)
+    for replay in (False, True):
+        for _ in range(6):
+            for stack in stacks:
+                stack.h.zero_()
+            torch.cuda.synchronize()
+            for stack, h, s, graph in zip(stacks, inputs, streams, graphs):
+                with torch.cuda.stream(s):
+                    if replay:
+                        graph.replay()
+                    else:
+                        for _ in range(8):
+                            stack(h)
+            torch.cuda.synchronize()
+            for stack, w in zip(stacks, want):
+                assert torch.equal(stack.h.view(torch.int32), w.view(torch.int32))
