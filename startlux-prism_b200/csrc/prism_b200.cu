@@ -6,7 +6,6 @@
 #include <stdlib.h>
 #include <string.h>
 
-#include <atomic>
 #include <mutex>
 #include <unordered_map>
 
@@ -64,8 +63,10 @@ EncodeTiledFn encode_fn() {
 // of the kernel before them on the stream; each begins with pdl_trigger and reads another kernel's output, or writes
 // global memory, only after pdl_wait.  Off: plain launches (the two instructions are no-ops then).  The one-row
 // CUDA-core GEMM stays a plain launch: as a programmatic dependent (first weights requested before the wait) the
-// one-row pass measured 0.42 ms per four layers against 0.33.
-std::atomic<int> g_pdl{0};
+// one-row pass measured 0.42 ms per four layers against 0.33.  Each thread has its own switch: a caller that turns it on
+// around a pass must not turn another thread's launches into dependents (whose weights may just be written), nor put back
+// what another thread had set.
+thread_local int g_pdl = 0;
 
 template <class... KA, class... A>
 cudaError_t launch_dep(void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
@@ -78,7 +79,7 @@ cudaError_t launch_dep(void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, 
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = g_pdl.load(std::memory_order_relaxed) ? 1 : 0;
+    cfg.numAttrs = g_pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
 }
 
@@ -892,7 +893,11 @@ int pb_set_wait_limit_ns(unsigned long long ns) {
     return PB_OK;
 }
 
-int pb_set_pdl(int on) { return g_pdl.exchange(on ? 1 : 0); }
+int pb_set_pdl(int on) {
+    const int before = g_pdl;
+    g_pdl = on ? 1 : 0;
+    return before;
+}
 
 int pb_test_drop_loads(int on) {
     g_drop_loads = on ? 1 : 0;
@@ -932,7 +937,7 @@ int pb_w8a8_gemm(const int8_t* a, const float* a_s, const int8_t* w, const float
     if (!a || !w || !out || !n_rows || M <= 0 || N <= 0 || K <= 0 || split < 1) return PB_BAD_ARGUMENT;
     if (epi != PB_EPI_BF16 && epi != PB_EPI_ADD && epi != PB_EPI_I32 && epi != PB_EPI_F32) return PB_BAD_ARGUMENT;
     const int pdl_asked = pdl;                                     // the caller's own request keeps a row off the CUDA-core kernel
-    if (g_pdl.load(std::memory_order_relaxed) && M <= 64) pdl = 1;
+    if (g_pdl && M <= 64) pdl = 1;
     if (epi == PB_EPI_F32 && (gk != 32 || M > 64)) return PB_UNSUPPORTED_SHAPE;
     if (epi != PB_EPI_I32 && (!a_s || !w_s)) return PB_BAD_ARGUMENT;
     if (!aligned16(a) || !aligned16(w)) return PB_BAD_ARGUMENT;

@@ -37,6 +37,22 @@ def test_operators_refuse_cpu_tensors(lib):
                   torch.tensor([4], dtype=torch.int32), 64)
 
 
+def test_pdl_switch_belongs_to_its_thread(lib):
+    """Two threads that each save, set and put back the switch around a pass, one inside the other's: neither sees the
+    other's setting, and nothing stays on."""
+    import threading
+    seen = []
+    assert lib.pb_set_pdl(1) == 0
+    try:
+        t = threading.Thread(target=lambda: seen.extend([lib.pb_set_pdl(1), lib.pb_set_pdl(0), lib.pb_set_pdl(0)]))
+        t.start()
+        t.join()
+        assert seen == [0, 1, 0]
+    finally:
+        assert lib.pb_set_pdl(0) == 1
+    assert lib.pb_set_pdl(0) == 0
+
+
 class _Recorder:
     """The library with every launch replaced by a note of its arguments."""
 
