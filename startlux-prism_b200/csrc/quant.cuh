@@ -616,11 +616,13 @@ fold_kernel(float* __restrict__ h, long ldh, const int32_t* __restrict__ slots, 
     }
 }
 
-// fold + rows_q8 of the same rows in one launch (few rows: each of the two is about a launch's latency): a CTA finishes its
-// row's deferred add, stores the residual and quantizes it from registers.  The operations of the two kernels on the same
-// values in the same order: the same bits.  One row per CTA keeps 2 * S independent 16-byte loads per thread in flight
-// (8 inputs a thread up to 8192 columns).  Four layers at 16 rows: see LinearStack.
-template <int VPT, bool FULL>
+// fold + rows_q8 of the same rows in one launch: a CTA finishes its row's deferred add, stores the residual and quantizes it
+// from registers.  The operations of the two kernels on the same values in the same order: the same bits.  Bound by the
+// bytes of the slots and the residual from about 200 rows on, by a launch's latency below; one row per CTA, eight columns a
+// thread, keeps 2 * S independent 16-byte loads per thread in flight.  us, two launches -> one, 5120 columns, buffers rotated
+// beyond L2 from 900 rows on: one slot, 16 rows 5.2 -> 3.0, 64 rows 5.6 -> 3.1, 1024 rows 17.2 -> 16.3, 4096 rows 64.8 -> 63.4;
+// four slots, 16 rows 5.7 -> 3.5.  Never behind with one slot; with two, up to 5 % at 4096 rows (78.9 -> 82.7).
+template <bool FULL>
 __global__ void __launch_bounds__(1024)
 fold_rows_q8_kernel(float* __restrict__ h, long ldh, const int32_t* __restrict__ slots, long slot_stride, int S,
                     const float* __restrict__ a_s, const float* __restrict__ w_s, int8_t* __restrict__ q,
@@ -630,43 +632,36 @@ fold_rows_q8_kernel(float* __restrict__ h, long ldh, const int32_t* __restrict__
     pdl_wait();
     const long r = blockIdx.x;
     if (r >= *n_rows) return;
-    const int nvec = N >> 3;
+    const int c = threadIdx.x;
+    const bool in = c < (N >> 3);
     const float sa = a_s[r];                                       // read before this row's new scale is written
-    float v[VPT][8];
+    float v[8];
     float amax = 0.0f;
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-        const int c = threadIdx.x + i * blockDim.x;
-        if (c < nvec) {
-            float* hp = h + r * ldh + (long)c * 8;
-            const float4 a = *(const float4*)hp, b = *(const float4*)(hp + 4);
-            int4 t0 = make_int4(0, 0, 0, 0), t1 = t0;
+    if (in) {
+        float* hp = h + r * ldh + (long)c * 8;
+        const float4 a = *(const float4*)hp, b = *(const float4*)(hp + 4);
+        int4 t0 = make_int4(0, 0, 0, 0), t1 = t0;
 #pragma unroll 4
-            for (int p = 0; p < S; ++p) {
-                const int4* pp = (const int4*)(slots + p * slot_stride + r * N + (long)c * 8);
-                const int4 x0 = __ldcs(pp), x1 = __ldcs(pp + 1);
-                t0.x += x0.x; t0.y += x0.y; t0.z += x0.z; t0.w += x0.w;
-                t1.x += x1.x; t1.y += x1.y; t1.z += x1.z; t1.w += x1.w;
-            }
-            const float4 w0 = __ldg((const float4*)(w_s + c * 8)), w1 = __ldg((const float4*)(w_s + c * 8 + 4));
-            v[i][0] = __fadd_rn(a.x, scale2(t0.x, sa, w0.x)); v[i][1] = __fadd_rn(a.y, scale2(t0.y, sa, w0.y));
-            v[i][2] = __fadd_rn(a.z, scale2(t0.z, sa, w0.z)); v[i][3] = __fadd_rn(a.w, scale2(t0.w, sa, w0.w));
-            v[i][4] = __fadd_rn(b.x, scale2(t1.x, sa, w1.x)); v[i][5] = __fadd_rn(b.y, scale2(t1.y, sa, w1.y));
-            v[i][6] = __fadd_rn(b.z, scale2(t1.z, sa, w1.z)); v[i][7] = __fadd_rn(b.w, scale2(t1.w, sa, w1.w));
-            *(float4*)hp = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
-            *(float4*)(hp + 4) = make_float4(v[i][4], v[i][5], v[i][6], v[i][7]);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(v[i][e]));
+        for (int p = 0; p < S; ++p) {
+            const int4* pp = (const int4*)(slots + p * slot_stride + r * N + (long)c * 8);
+            const int4 x0 = __ldcs(pp), x1 = __ldcs(pp + 1);
+            t0.x += x0.x; t0.y += x0.y; t0.z += x0.z; t0.w += x0.w;
+            t1.x += x1.x; t1.y += x1.y; t1.z += x1.z; t1.w += x1.w;
         }
+        const float4 w0 = __ldg((const float4*)(w_s + c * 8)), w1 = __ldg((const float4*)(w_s + c * 8 + 4));
+        v[0] = __fadd_rn(a.x, scale2(t0.x, sa, w0.x)); v[1] = __fadd_rn(a.y, scale2(t0.y, sa, w0.y));
+        v[2] = __fadd_rn(a.z, scale2(t0.z, sa, w0.z)); v[3] = __fadd_rn(a.w, scale2(t0.w, sa, w0.w));
+        v[4] = __fadd_rn(b.x, scale2(t1.x, sa, w1.x)); v[5] = __fadd_rn(b.y, scale2(t1.y, sa, w1.y));
+        v[6] = __fadd_rn(b.z, scale2(t1.z, sa, w1.z)); v[7] = __fadd_rn(b.w, scale2(t1.w, sa, w1.w));
+        *(float4*)hp = make_float4(v[0], v[1], v[2], v[3]);
+        *(float4*)(hp + 4) = make_float4(v[4], v[5], v[6], v[7]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(v[e]));
     }
     amax = block_max(amax, red);
     const float scale = fdiv<FULL>(fmaxf(amax, 1e-10f), 127.0f);
     const float rcp = __fdiv_rn(1.0f, scale);
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-        const int c = threadIdx.x + i * blockDim.x;
-        if (c < nvec) *(uint2*)(q + r * N + (long)c * 8) = quant8<FULL>(v[i], scale, rcp);
-    }
+    if (in) *(uint2*)(q + r * N + (long)c * 8) = quant8<FULL>(v, scale, rcp);
     if (threadIdx.x == 0) s[r] = scale;
 }
 

@@ -100,7 +100,7 @@ def test_fold_odd(dev):
 @pytest.mark.parametrize("T,N,S,live", [(1, 8, 1, 1), (16, 5120, 7, 13), (3, 8192, 2, 3), (5, 8200, 3, 5), (64, 264, 8, 64)])
 def test_fold_rows_q8(dev, T, N, S, live):
     """The one-launch form against fold and rows_q8 of the oracle: residual, int8 rows and scales alike, rows >= live
-    untouched; either side of 8192 columns (one or eight vectors a thread), the scales written over the add's own."""
+    untouched; either side of 8192 columns (one launch or two), the scales written over the add's own."""
     g = torch.Generator().manual_seed(N)
     slots = torch.randint(-10 ** 6, 10 ** 6, (S, T, N), generator=g, dtype=torch.int32)
     sa, sw = torch.rand(T, generator=g) * 1e-2, torch.rand(N, generator=g) * 1e-3
@@ -113,6 +113,33 @@ def test_fold_rows_q8(dev, T, N, S, live):
     assert same(hd, ref)
     assert same(q[:live], rq[:live]) and same(sd[:live], rs[:live, 0]) and same(sd[live:], sa[live:])
     assert bool((q[live:] == 99).all())
+
+
+@pytest.mark.parametrize("T,N", [(300, 1032), (2, 8192), (6, 8208)])
+def test_fold_rows_q8_strides(dev, T, N):
+    """A residual that is a column slice of a wider buffer and slots with more rows than the call takes; and what does not
+    fit is refused before anything is launched."""
+    S = 2
+    g = torch.Generator().manual_seed(T + N)
+    slots = torch.randint(-10 ** 6, 10 ** 6, (S, T + 3, N), generator=g, dtype=torch.int32)
+    sa, sw = torch.rand(T, generator=g) * 1e-2, torch.rand(N, generator=g) * 1e-3
+    wide = torch.randn(T, N + 20, generator=g)
+    ref = oracle.fold(wide[:, :N].numpy(), slots[:, :T].numpy(), sa.numpy(), sw.numpy())
+    rq, rs = oracle.quant_rows(ref)
+    wd, sd = wide.to(dev), torch.empty(T, device=dev)
+    q = torch.empty(T, N, dtype=torch.int8, device=dev)
+    sld, pend, nr = slots.to(dev), w8a8.Deferred(S, sa.to(dev), sw.to(dev)), n_rows(T, dev)
+    quant.fold_rows_q8(wd[:, :N], sld, pend, q, sd, nr, T)
+    assert same(wd[:, :N].contiguous(), ref) and same(wd[:, N:].contiguous(), wide[:, N:].contiguous())
+    assert same(q, rq) and same(sd, rs[:, 0])
+    kept = wd.clone()
+    for bad in (dict(s=sd[:T - 1]), dict(q=q[:T - 1]), dict(h=wd[:T - 1, :N]), dict(parts=sld[:, :T - 1]), dict(parts=sld[:1]),
+                dict(parts=torch.empty(S, T, N + 8, dtype=torch.int32, device=dev)[..., :N]), dict(pend=pend._replace(w_s=pend.w_s[:N - 1])),
+                dict(pend=pend._replace(a_s=pend.a_s[:T - 1]))):
+        arg = {"h": wd[:, :N], "parts": sld, "pend": pend, "q": q, "s": sd, **bad}
+        with pytest.raises(RuntimeError):
+            quant.fold_rows_q8(arg["h"], arg["parts"], arg["pend"], arg["q"], arg["s"], nr, T)
+    assert same(wd, kept)
 
 
 @pytest.mark.parametrize("T,K,live", [(300, 5120, 290), (1000, 2560, 1000), (260, 17408, 257), (512, 264, 512)])
