@@ -485,37 +485,61 @@ int launch_g32_mma(const int8_t* a, const int8_t* w, const w8a8::SwapArgs& p, cu
     return PB_OK;
 }
 
-// Which one (measured at 1 to 1000 rows on 1792 ... 34816 x 5120, 5120 x 8704 / 17408 and the 248320 x 5120 head; us, tcgen05
-// against mma.sync).
-//   - up to 16 rows: one warp per 16 weight rows x 8 rows in a CTA of its own, so that a few weight rows still cover the SMs
-//     (5120 x 5120: 12.8 against 11.1 at 8 rows, 13.5 against 12.1 at 12); with N / 16 warps eight per SM already (`wide`), CTAs that
-//     share the activations (34816 rows, 16 rows: 39.0 us against 50.5 without).  Between them, where the 128-row tiles of
-//     tcgen05 alone are one nearly full wave, that kernel (17408 rows, 12 rows: 21.7 against 26.8).
-//   - 17 to 64 rows, not wide: tcgen05 in row blocks of 16 while they fit one wave (5120 x 5120 at 24 rows 18.9 against 19.8), else
-//     of 32 (7168 at 40 rows 30.1 against 35.5); at 33 rows up against few weight rows warps again (5120 at 56: 29.5 against 26.4).
+// Which one.  Measured at 1 to 1000 rows on 256 ... 57344 weight rows x 512 ... 17408 and heads of 19200 ... 250000 rows; us of one
+// launch with weights from HBM, tcgen05 against mma.sync where nothing else is said.  Above 1000 rows (to 8192, on fifteen shapes) nothing is slower than
+// the tcgen05 kernel that ran everything before.
+//   - up to 8 rows the line is how the weight rows fill the SMs, since a last, partial round takes almost as long as a whole one: 80
+//     of them per SM are resident as five CTAs of 16 (`r16` rounds), 128 as four CTAs of 32 or as one tcgen05 tile (`r32`).
+//     CTAs of 16 while they are one round (8192 x 5120: 15.8 against 12.1) or leave less idle than those of 32 (22016 x 5120: 26.9,
+//     28.4 with 32, 33.0 on tcgen05; at three rounds or more only from K = 4096 on: 28672 x 1024 11.7 against 10.7 with 32);
+//     tcgen05 where its tiles are one wave at least three quarters full (16384 x 5120: 18.1 against 19.0) or, K long enough to hide
+//     its set-up, two nearly full ones (32000 x 4096: 29.6 against 30.0; 34816 x 5120: 35.7 against 36.4; x 2048: 20.0 against 18.6),
+//     and for long K (8192 measured) in every partial wave (14208 x 8192: 24.7 against 26.0; 28672: 49.8 against 52.3);
+//     else CTAs of 32 (12288 x 4096: 12.9, 18.1 with 16, 14.1 on tcgen05; 51200 x 5120: 51.6 against 55.2 and 51.7).
+//   - 9 to 16 rows: two warps per 16 weight rows while four such CTAs per SM take them all (9216 x 5120: 18.8 against 15.8); tcgen05
+//     while its tiles are one wave (12288 x 4096: 16.7 against 21.6); then CTAs of 64 weight rows up to one round of three per SM
+//     and from two rounds of CTAs of 128 on (24576 x 5120: 32.3, 34.1 with 128; 62080: 69.0, 80.4), between the two CTAs of 128
+//     (34816 x 5120: 39.4, 44.2 with 64, 40.9 on tcgen05) or, for long K, tcgen05 again (34816 x 8192: 58.0 against 63.5).
+//   - 17 to 64 rows, weight tiles within one wave: tcgen05 in row blocks of 16 while they fit one wave (5120 x 5120 at 24 rows 18.9
+//     against 19.8), else of 32 (7168 at 40 rows 30.1 against 35.5); at 33 rows up against few weight rows warps again (5120 at 56:
+//     29.5 against 26.4).
 //   - more, or wide: warps of 32 weight rows, whose two tiles share every activation operand and scale read from shared memory -
-//     its bandwidth is the bound at one tile per warp (head at 48 rows: 379 us against 418) - on CTA tiles of 64 x 64, 64 x 48
-//     or 128 x 24, whichever leaves the least idle in the last round of CTAs per SM (7168 at 220 rows: 86.0 against 73.4); but
-//     where that is more than one round of the smallest tile and tcgen05's row blocks of 32 are one wave, these (5120 x 17408 at 72 rows
-//     87.8 against 92.5).  A last row block of at most eight rows costs little: it may lie a seventh over the wave.
+//     its bandwidth is the bound at one tile per warp (head at 48 rows: 379 us against 418).  Up to 24 rows CTAs of 128 x 24
+//     (32000 x 4096: 40.9 against 33.8), up to 48 of 64 x 48 while three per SM take the weight rows (20480 x 5120: 64.6, 72.0 with
+//     128 x 48, 55.0); above on 64 x 64, 64 x 48 or 128 x 24, whichever leaves the least idle in the last round of CTAs per SM
+//     (7168 at 220 rows: 86.0 against 73.4); but where that is more than one round of the smallest tile and tcgen05's row blocks
+//     of 32 are one wave, these (5120 x 17408 at 72 rows 87.8 against 92.5).  A last row block of at most eight rows costs little: it
+//     may lie a seventh over the wave.
 int launch_g32_any(const int8_t* a, const int8_t* w, const w8a8::SwapArgs& p, cudaStream_t st) {
     const int M = p.M, N = p.N;
     const long sms = sm_count(), tiles = (N + 127) / 128;
-    const bool wide = N >= 16 * 8 * sms;
+    const bool wide = N >= 16 * 8 * sms, deep = p.K >= 8192;
     const bool can16 = w8a8::G32<16>::stages_for(p.K, 16) >= 3, can32 = w8a8::G32<32>::stages_for(p.K, 32) >= 3;
+    if (M <= 8) {
+        const long r16 = (N + 80 * sms - 1) / (80 * sms), r32 = (N + 128 * sms - 1) / (128 * sms), all32 = r32 * 128 * sms;
+        const bool tc = r32 == 1 ? tiles * 4 > sms * 3 || deep : r32 == 2 && (deep ? r16 > 2 : p.K >= 4096 && N * 6L > all32 * 5);
+        if (r16 == 1) return launch_g32_mma<1, 1, 1, 1, 4, 3>(a, w, p, st);
+        if (tc && can16) return launch_g32<16>(a, w, p, st);
+        if (r16 * 80 < r32 * 128 && N * 8L <= all32 * 7 && (r16 == 2 || p.K >= 4096))
+            return launch_g32_mma<1, 1, 1, 1, 4, 3>(a, w, p, st);
+        return launch_g32_mma<1, 1, 2, 1, 2, 4>(a, w, p, st);
+    }
     if (M <= 16) {
-        if (!wide && tiles * 4 > sms * 3 && tiles <= sms && can16) return launch_g32<16>(a, w, p, st);
-        if (M <= 8) return wide ? launch_g32_mma<1, 1, 2, 1, 2, 4>(a, w, p, st) : launch_g32_mma<1, 1, 1, 1, 4, 3>(a, w, p, st);
-        if (!wide) return launch_g32_mma<1, 1, 1, 2, 4, 3>(a, w, p, st);
-        return N >= 64 * 8 * sms ? launch_g32_mma<2, 2, 2, 1, 2, 3>(a, w, p, st) : launch_g32_mma<2, 2, 4, 1, 1, 3>(a, w, p, st);
+        if (N <= 4 * 16 * sms) return launch_g32_mma<1, 1, 1, 2, 4, 3>(a, w, p, st);
+        const bool few = N <= 3 * 64 * sms;
+        if ((tiles <= sms || (deep && !few && tiles <= 2 * sms)) && can16) return launch_g32<16>(a, w, p, st);
+        return few || N > 3 * 128 * sms ? launch_g32_mma<2, 2, 2, 1, 2, 3>(a, w, p, st)
+                                        : launch_g32_mma<2, 2, 4, 1, 1, 3>(a, w, p, st);
     }
     if (tiles * ((M + 15) / 16) <= sms && can16) return launch_g32<16>(a, w, p, st);
+    if (M <= 32 && tiles <= sms && can32) return launch_g32<32>(a, w, p, st);
     if (M <= 64 && !wide) {
-        if ((M <= 32 || tiles * 3 > sms) && can32) return launch_g32<32>(a, w, p, st);
+        if (tiles * 3 > sms && can32) return launch_g32<32>(a, w, p, st);
         return launch_g32_mma<2, 1, 2, 2, 2, 4>(a, w, p, st);
     }
+    if (M <= 24) return launch_g32_mma<3, 2, 4, 1, 1, 3>(a, w, p, st);
     if (M <= 32) return launch_g32_mma<4, 2, 4, 1, 1, 3>(a, w, p, st);
-    if (M <= 48) return launch_g32_mma<6, 2, 4, 1, 1, 3>(a, w, p, st);
+    if (M <= 48) return N <= 3 * 64 * sms ? launch_g32_mma<3, 2, 2, 2, 1, 4>(a, w, p, st) : launch_g32_mma<6, 2, 4, 1, 1, 3>(a, w, p, st);
     // rounds of CTAs per SM x the tile's 16 x 8 units x its measured time per unit
     const auto cost = [&](int rows, int mc, int time) {
         return ((long)((N + rows - 1) / rows) * ((M + mc - 1) / mc) + sms - 1) / sms * (rows / 16) * (mc / 8) * time;

@@ -15,8 +15,8 @@
 //     memory, and never waits on a pipeline stage: the stages go back to the producer when their MMAs have completed.
 // Roles: warp 0 = TMA producer (one thread), warps 1 and 2 = MMA issuers (one thread each; warp 1 owns the tensor
 // memory), warps 3..10 = epilogue: two warps per lane quarter, each with RW = NB / 2 of the CTA's activation rows.
-// NB = 16 or 32: row blocks of that many activation rows in grid.z, for the row counts whose blocks all fit one wave of CTAs
-// (each block re-reads the weights from L2); everything else runs on w8a8_g32_mma.cuh.
+// NB = 16 or 32: row blocks of that many activation rows in grid.z, mostly for sizes whose blocks fit one wave of CTAs (each
+// block re-reads the weights from L2; launch_g32_any has the lines); everything else runs on w8a8_g32_mma.cuh.
 #pragma once
 #include "w8a8_gemm.cuh"
 

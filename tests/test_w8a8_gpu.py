@@ -365,6 +365,39 @@ def test_groups_of_32_every_tile(dev, M, N, K, live):
         assert np.array_equal(f.cpu().numpy()[:live], ref[:live]) and bool((f[live:] == 7.0).all())
 
 
+@pytest.mark.parametrize("M,N,K,live", [(8, 100, 3456, 8), (8, 13000, 2176, 7), (5, 20500, 3456, 5), (12, 130, 3456, 12),
+                                        (16, 19000, 1664, 15), (13, 28500, 1152, 13), (20, 19000, 1152, 20), (30, 19000, 1152, 30),
+                                        (44, 19000, 1408, 44), (40, 28500, 1152, 37), (56, 5120, 2176, 56), (64, 19000, 1408, 64),
+                                        (220, 7168, 1408, 215), (12, 17000, 2432, 12), (3, 32500, 4096, 3), (9, 28500, 8192, 9),
+                                        (4, 12000, 8192, 4), (30, 7168, 2432, 30)])
+def test_groups_of_32_long_k(dev, M, N, K, live):
+    """Per-32 groups, a K that takes each tile of the dispatch several times around its ring of stages and ends inside one (and
+    tcgen05 where K or the weight rows call for it), out a column slice at an odd offset of a buffer with an odd row
+    stride.  The tiles' first, last and 200 other weight rows against the oracle: stores, residual adds and the head's chain."""
+    a, w, sa, sw = rand_w8a8(M, N, K, seed=M + N + K, groups=K // 32)
+    g = torch.Generator().manual_seed(K)
+    at = torch.cat([torch.arange(min(N, 70)), torch.randint(0, N, (200,), generator=g), torch.arange(max(N - 70, 0), N)])
+    args = (a.numpy(), sa.numpy(), w[at].numpy(), sw[at].numpy(), 32)
+    dargs = (a.to(dev), sa.to(dev), w.to(dev), sw.to(dev))
+    nr = n_rows(live, dev)
+    wide = torch.full((M, N + 8), 3.0, dtype=torch.bfloat16, device=dev)
+    w8a8.gemm(*dargs, wide[:, 5:5 + N], nr, 32)
+    got = wide.cpu()
+    ref = oracle.w8a8_gemm(*args, 0, live)
+    assert np.array_equal(np_bits(got[:live, 5 + at]), ref[:live]), first_diff(np_bits(got[:live, 5 + at]), ref[:live])
+    assert bool((got[live:] == 3).all()) and bool((got[:, :5] == 3).all()) and bool((got[:, 5 + N:] == 3).all())
+    h = torch.randn(M, N + 3, generator=g)
+    hd = h.to(dev)
+    w8a8.gemm(*dargs, hd[:, 1:1 + N], nr, 32, epi=1)
+    ref = oracle.w8a8_gemm(*args, 1, live, out=h[:, 1 + at].numpy())
+    assert same(hd.cpu()[:, 1 + at], ref) and same(hd.cpu()[:, 1 + N:], h[:, 1 + N:])
+    if M <= 64:
+        f = torch.full((M, N), 7.0, device=dev)
+        w8a8.gemm(*dargs, f, nr, 32, epi=w8a8.EPI_F32)
+        ref = oracle.w8a8_gemm(*args, 4, live)
+        assert same(f.cpu()[:live, at], ref[:live]) and bool((f[live:] == 7).all())
+
+
 @pytest.mark.parametrize("M,N,K", [(8, 640, 1024), (12, 17408, 256), (40, 19000, 256), (56, 5120, 512)])
 def test_dependent_reads_weight_scales_after_the_wait(dev, M, N, K):
     """pdl=True and per-32 groups: the kernel before (a fold, which lets its dependents start at once and then takes its
