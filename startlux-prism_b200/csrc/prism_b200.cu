@@ -639,20 +639,26 @@ int launch_w4a8_mma(const w4a8::GemvArgs& p, cudaStream_t st) {
     return PB_OK;
 }
 
-// Which one: measured on 5120 / 6144 / 34816 x 5120 (Q4_K) and 1024 x 5120, 5120 x 17408 (Q6_K), one launch, weights from HBM.
-// With N / 16 warps already eight per SM (`wide`) every warp walks through the whole of K; below that K is split over
-// the CTA's warps and a CTA takes 16 weight rows, so that 5120 rows still are two CTAs per SM (Q4_K, 8 rows: wide
-// 21.4 us whole against 26.8 split on 34816 rows, 10.3 against 7.0 on 5120).  More rows than 16 take their activation rows in blocks of 16
-// there (14.9 us against 15.8 at 32 rows in one block).
+// Which one: measured at 2 to 32 rows on 1024 ... 40960 weight rows x 512 ... 8192, one launch, weights from HBM.
+// Q4_K: K split over the CTA's four warps and 16 weight rows per CTA while three such CTAs per SM hold all weight rows (`fit`; 8 rows
+// of 6144 x 5120 7.1 us against 10.3 with whole-K warps).  Beyond that a second, partial round of them costs more than whole-K
+// warps on 64 or 128 weight rows do - at once for short K, of which four warps have little to share (14336 x 512, 2 rows: 5.8 against
+// 3.6; 16 rows: 6.8 against 4.8), for longer K from the third round on (2 rounds: 8192 x 8192, 8 rows 14.0 against 15.2, 11008 x 2048,
+// 16 rows 9.1 against 9.6; 3: 14336 x 5120, 8 rows 14.4 against 13.1).  More rows than 16 take 16 at a time there, so their
+// CTAs are twice as many, and 32 in one CTA beyond (6144 x 5120 15.7 against 16.2; 8192 x 5120 20.7 against 16.4).
+// Q6_K: 16 weight rows per CTA while that is one CTA per SM, up to 8 rows two (3072 x 4096, 4 rows: 6.3 against 7.1 with 32 a CTA;
+// but 4736 x 512 2.6 against 2.4: short K again).
 template <int KIND>
 int launch_w4a8_few(const w4a8::GemvArgs& p, cudaStream_t st) {
+    const int sms = sm_count();
     if (KIND == w4a8::KIND_Q4K) {
-        const bool wide = p.N >= 16 * 8 * sm_count();
-        if (p.M <= 8) return wide ? launch_w4a8_mma<KIND, 1, 1, 4, 1, 4>(p, st) : launch_w4a8_mma<KIND, 1, 1, 1, 4, 3>(p, st);
-        if (!wide) return launch_w4a8_mma<KIND, 2, 1, 1, 4, 2>(p, st);
+        const int fit = 3 * 16 * sms;
+        if (p.M <= 8) return p.N <= fit || (p.N <= 2 * fit && p.K > 2048) ? launch_w4a8_mma<KIND, 1, 1, 1, 4, 3>(p, st)
+                                                                         : launch_w4a8_mma<KIND, 1, 1, 4, 1, 4>(p, st);
+        if (p.N <= fit || (p.M <= 16 && p.N <= 2 * fit && p.K > 1024)) return launch_w4a8_mma<KIND, 2, 1, 1, 4, 2>(p, st);
         return p.M <= 16 ? launch_w4a8_mma<KIND, 2, 2, 4, 1, 3>(p, st) : launch_w4a8_mma<KIND, 4, 1, 4, 2, 2>(p, st);
     }
-    if (p.N <= 16 * sm_count())
+    if (p.N <= 16 * sms || (p.M <= 8 && p.N <= 32 * sms && p.K > 1024))
         return p.M <= 16 ? launch_w4a8_mma<KIND, 1, 1, 1, 4, 4>(p, st) : launch_w4a8_mma<KIND, 2, 1, 1, 4, 3>(p, st);
     if (p.M <= 8) return launch_w4a8_mma<KIND, 1, 1, 2, 4, 2>(p, st);
     return p.M <= 16 ? launch_w4a8_mma<KIND, 2, 2, 2, 4, 2>(p, st) : launch_w4a8_mma<KIND, 4, 1, 4, 2, 2>(p, st);
