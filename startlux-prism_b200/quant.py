@@ -280,17 +280,16 @@ def fold_rows_q8(h, parts, pending, q, s, n, T):
         return rows_q8(h, None, q, s, n, T)
     if pending.parts is not None:
         parts = pending.parts
+    S, a_s, w_s = pending.n, pending.a_s, pending.w_s
     _lib.need_cuda(h, parts, q, s, n)
-    if h.dtype != torch.float32 or parts.dtype != torch.int32 or parts.shape[2] != N or h.stride(1) != 1 \
-            or q.shape[1] != N or not q.is_contiguous() or q.dtype != torch.int8:
-        raise RuntimeError("fold_rows_q8: h fp32 [T, N], parts int32 [S, rows, N], q int8 [T, N]")
-    if parts.stride(1) != N or parts.stride(2) != 1 or parts.shape[0] < pending.n or min(h.shape[0], parts.shape[1], q.shape[0]) < T:
-        raise RuntimeError(f"fold_rows_q8: h, q and each of {pending.n} slots need {T} rows, the slots' rows contiguous")
-    for name, t, need in (("s", s, T), ("the pending a_s", pending.a_s, T), ("the pending w_s", pending.w_s, N)):
-        if t.dtype != torch.float32 or not t.is_contiguous() or t.numel() < need:
-            raise RuntimeError(f"fold_rows_q8: {name} must be contiguous fp32 with at least {need} elements")
-    rc = _lib.lib().pb_fold_rows_q8(_lib.ptr(h), h.stride(0), _lib.ptr(parts), parts.stride(0), pending.n,
-                                    _lib.ptr(pending.a_s), _lib.ptr(pending.w_s), _lib.ptr(q), _lib.ptr(s), _lib.ptr(n), T, N,
-                                    _lib.stream())
+    f32, pst = torch.float32, parts.stride(0)
+    if h.dtype != f32 or s.dtype != f32 or a_s.dtype != f32 or w_s.dtype != f32 or parts.dtype != torch.int32 \
+            or q.dtype != torch.int8 or h.stride(1) != 1 or not q.is_contiguous() or parts.stride() != (pst, N, 1):
+        raise RuntimeError("fold_rows_q8: h fp32 [T, N], parts int32 [S, rows, N], q int8 [T, N], scales fp32")
+    (ps, pr, pn), (qr, qn) = parts.shape, q.shape
+    if pn != N or qn != N or ps < S or min(pr, qr, h.shape[0], s.numel(), a_s.numel()) < T or w_s.numel() < N:
+        raise RuntimeError(f"fold_rows_q8: h, q, s, a_s and each of {S} slots need {T} rows, w_s {N} columns")
+    rc = _lib.lib().pb_fold_rows_q8(h.data_ptr(), h.stride(0), parts.data_ptr(), pst, S, a_s.data_ptr(), w_s.data_ptr(),
+                                    q.data_ptr(), s.data_ptr(), n.data_ptr(), T, N, _lib.stream())
     if rc:
-        _lib.check(rc, f"fold_rows_q8 T={T} N={N} S={pending.n}")
+        _lib.check(rc, f"fold_rows_q8 T={T} N={N} S={S}")

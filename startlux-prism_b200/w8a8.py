@@ -230,7 +230,7 @@ def gemm(a, a_s, w, w_s, out, n_rows, gk, epi=0, outs=None, cfg=None, slots=None
     ws = counters = None
     if split > 1:
         ws, counters = (scratch.ws, scratch.counters) if scratch else _workspace(a.device)
-        if scratch and _lib.lib().pb_w8a8_counters(M, N) > counters.numel():
+        if scratch and -(-N // 128) > counters.numel():       # one per tile of 128 weight rows
             split = 1
         while split > 1 and _lib.lib().pb_w8a8_workspace_bytes(M, N, split) > ws.numel():
             split -= 1
