@@ -82,8 +82,11 @@ class LinearStack:
         # (pb_set_pdl): a GEMM's set-up and first weight reads run while the quantizer before it still works, a
         # quantizer's launch hides behind the GEMM's tail: 0.364 -> 0.332 ms per four-layer pass at 16 rows, 0.428 ->
         # 0.402 at 64, as a replayed graph.  One row too, on the tensor-core kernel then: 0.318 ms with the CUDA-core GEMM's
-        # plain launches, 0.297 as a chain (0.42 with that GEMM as a dependent).  PRISM_B200_PDL=0 keeps plain launches.
-        self.pdl = n == 1 and M <= w8a8.FEW_ROWS and os.environ.get("PRISM_B200_PDL", "1") != "0"
+        # plain launches, 0.297 as a chain (0.42 with that GEMM as a dependent) - unless the layer's weights are so few that
+        # launches are all there is to hide: four layers of 11 M weights 0.104 ms plain against 0.112, of 24 M 0.113 against
+        # 0.116, of 34 M 0.138 against 0.126, of 50 M 0.144 against 0.134.  PRISM_B200_PDL=0 keeps plain launches.
+        few = sum(w.shape[0] * w.shape[1] for lw in layers for w, _ in lw.values()) < 28_000_000 * len(layers)
+        self.pdl = (n == 1 and M <= w8a8.FEW_ROWS and not (M == 1 and few) and os.environ.get("PRISM_B200_PDL", "1") != "0")
         # a few-row pass adds its K splits in memory of its own (2 to 4 MB at the 27B shapes): the passes of two stacks may
         # overlap on two streams, and a pass can be captured unrun
         self.scratch = None

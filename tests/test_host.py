@@ -70,6 +70,33 @@ class _Recorder:
         return launch
 
 
+class _Weights:
+    """A weight matrix's shape: no memory is touched."""
+
+    def __init__(self, n, k):
+        self.shape, self.dtype = (n, k), torch.int8
+
+    def is_contiguous(self):
+        return True
+
+    def data_ptr(self):
+        return 4096
+
+
+def test_one_row_chain_needs_weights_to_hide(lib):
+    """One row: a chain of dependent launches where a layer's weights are worth prefetching, plain launches (the CUDA-core
+    GEMM) below that; more rows: always a chain."""
+    from prism_b200 import linear_stack as LS
+
+    def chained(M, hid, kv, ffn):
+        shapes = {"qkv": (hid + 2 * kv, hid), "o": (hid, hid), "gate_up": (2 * ffn, hid), "down": (hid, ffn)}
+        layer = {name: (_Weights(n, k), torch.ones(n)) for name, (n, k) in shapes.items()}
+        return LS.LinearStack([layer], M, torch.device("cpu"), None, hid, hid, kv, ffn).pdl
+    assert chained(1, 5120, 1024, 17408) and chained(1, 1792, 256, 4864)
+    assert not chained(1, 1024, 256, 2816) and not chained(1, 1536, 256, 4096)
+    assert chained(2, 1024, 256, 2816) and chained(64, 512, 128, 1408) and not chained(65, 5120, 1024, 17408)
+
+
 @pytest.mark.parametrize("M", [1, 2, 16, 64])
 def test_few_row_stacks_share_no_workspace(lib, monkeypatch, M):
     """Two stacks of the 27B shapes may have their passes in flight on two streams: a product that splits K inside the
@@ -82,17 +109,8 @@ def test_few_row_stacks_share_no_workspace(lib, monkeypatch, M):
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
     monkeypatch.setattr(w8a8, "_WORKSPACE", {})
 
-    class Weights:                                  # shapes only: no memory is touched
-        def __init__(self, n, k):
-            self.shape, self.dtype = (n, k), torch.int8
-
-        def is_contiguous(self):
-            return True
-
-        def data_ptr(self):
-            return 4096
     shapes = {"qkv": (7168, 5120), "o": (5120, 5120), "gate_up": (34816, 5120), "down": (5120, 17408)}
-    layers = [{name: (Weights(n, k), torch.ones(n)) for name, (n, k) in shapes.items()}]
+    layers = [{name: (_Weights(n, k), torch.ones(n)) for name, (n, k) in shapes.items()}]
     used = []
     for _ in range(2):
         stack = LS.LinearStack(layers, M, torch.device("cpu"))
