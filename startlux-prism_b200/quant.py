@@ -278,18 +278,19 @@ def fold_rows_q8(h, parts, pending, q, s, n, T):
     if not pending or pending.sync is not None or N % 8 or N > 65536:
         fold(h, parts, pending, n, T)
         return rows_q8(h, None, q, s, n, T)
-    if pending.parts is not None:
-        parts = pending.parts
-    S, a_s, w_s = pending.n, pending.a_s, pending.w_s
-    _lib.need_cuda(h, parts, q, s, n)
-    f32, pst = torch.float32, parts.stride(0)
+    S, a_s, w_s, own, _ = pending
+    if own is not None:
+        parts = own
+    if not (h.is_cuda and parts.is_cuda and q.is_cuda and s.is_cuda and n.is_cuda):
+        _lib.need_cuda(h, parts, q, s, n)
+    f32 = torch.float32
+    (hst, h1), (pst, p1, p2), (ps, pr, pn), (qr, qn) = h.stride(), parts.stride(), parts.shape, q.shape
     if h.dtype != f32 or s.dtype != f32 or a_s.dtype != f32 or w_s.dtype != f32 or parts.dtype != torch.int32 \
-            or q.dtype != torch.int8 or h.stride(1) != 1 or not q.is_contiguous() or parts.stride() != (pst, N, 1):
+            or q.dtype != torch.int8 or h1 != 1 or not q.is_contiguous() or p1 != N or p2 != 1 or pn != N or qn != N:
         raise RuntimeError("fold_rows_q8: h fp32 [T, N], parts int32 [S, rows, N], q int8 [T, N], scales fp32")
-    (ps, pr, pn), (qr, qn) = parts.shape, q.shape
-    if pn != N or qn != N or ps < S or min(pr, qr, h.shape[0], s.numel(), a_s.numel()) < T or w_s.numel() < N:
+    if ps < S or pr < T or qr < T or h.shape[0] < T or s.numel() < T or a_s.numel() < T or w_s.numel() < N:
         raise RuntimeError(f"fold_rows_q8: h, q, s, a_s and each of {S} slots need {T} rows, w_s {N} columns")
-    rc = _lib.lib().pb_fold_rows_q8(h.data_ptr(), h.stride(0), parts.data_ptr(), pst, S, a_s.data_ptr(), w_s.data_ptr(),
+    rc = _lib.lib().pb_fold_rows_q8(h.data_ptr(), hst, parts.data_ptr(), pst, S, a_s.data_ptr(), w_s.data_ptr(),
                                     q.data_ptr(), s.data_ptr(), n.data_ptr(), T, N, _lib.stream())
     if rc:
         _lib.check(rc, f"fold_rows_q8 T={T} N={N} S={S}")
