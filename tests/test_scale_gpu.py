@@ -88,7 +88,7 @@ def test_w8a8_at_scale(dev, name, M):
 @pytest.mark.parametrize("name,M", [("o", 2048), ("qkv", 2048), ("down", 256), ("o", 8192)])
 def test_w8a8_q8_0_groups_at_scale(dev, name, M):
     """Q8_0's own scale per 32 inputs on both operands (config 1 run with GK = 32) at prefill row counts: the fp32 sum
-    in group order (kernels/w8a8.py:64-76), row blocks of 32 per CTA.  64 sampled rows against the oracle, bf16 store
+    in group order (kernels/w8a8.py:64-76), on warps of 32 weight rows (csrc/w8a8_g32_mma.cuh).  64 sampled rows against the oracle, bf16 store
     and fp32 residual add, live < M; rows past live keep their poison."""
     N, K = SHAPES[name]
     G = K // 32
