@@ -423,10 +423,10 @@ int launch_swap(const int8_t* a, const float* a_s, const int8_t* w, const float*
     return PB_OK;
 }
 
-// Per-32 groups, up to 16 rows, one K slice, fewer weight tiles than SMs: how many activation rows a CTA owns (16, 8 or
-// 4).  Fewer rows per CTA = more CTAs on one weight tile, i.e. the per-group fp32 arithmetic (what bounds this kernel:
-// ncu shows the fp32 pipe saturated on the SMs in use) spread over more SMs; the smallest count whose grid still
-// fits the SMs at once.  PRISM_B200_GROWS forces 16 / 8 / 4.
+// Per-32 groups, up to 16 rows, one K slice on w8a8_swap_kernel, i.e. in comparison runs with PRISM_B200_G32=0 only: how many
+// activation rows a CTA owns (16, 8 or 4).  Fewer rows per CTA = more CTAs on one weight tile, i.e. the per-group fp32
+// arithmetic spread over more SMs; the smallest count whose grid still fits the SMs at once.  PRISM_B200_GROWS forces
+// 16 / 8 / 4 there.
 int grouped_rows_per_cta(int M, int N) {
     static const int forced = [] { const char* e = getenv("PRISM_B200_GROWS"); return e ? atoi(e) : 0; }();
     if (forced == 16 || forced == 8 || forced == 4) return forced;
@@ -445,7 +445,7 @@ int launch_g32(const int8_t* a, const int8_t* w, w8a8::SwapArgs p, cudaStream_t 
     if ((rc = tensor_map_kchunks(&tw, w, p.N, p.K, w8a8::BM))) return rc;
     if ((rc = tensor_map_kchunks(&tx, a, p.M, p.K, NB))) return rc;
     p.stages = C::stages_for(p.K, NB);
-    auto kern = w8a8::w8a8_g32_kernel<NB, NB / 2>;
+    auto kern = w8a8::w8a8_g32_kernel<NB>;
     if ((rc = set_smem(kern, 232448))) return rc;
     dim3 grid((p.N + w8a8::BM - 1) / w8a8::BM, 1, (p.M + NB - 1) / NB);
     cudaLaunchConfig_t cfg = {};
@@ -669,8 +669,9 @@ template <int MR>
 int launch_w4a8_gemv(int kind, const w4a8::GemvArgs& p, cudaStream_t st) {
     constexpr int R = w4a8::GEMV_R;
     const int grid = (p.N + 4 * R - 1) / (4 * R);                  // eight weight rows per CTA
-    auto split_k = kind == 0 ? w4a8::w4a8_gemv_q4k_kernel<MR, R, true> : w4a8::w4a8_gemv_q6k_kernel<MR, R, true>;
-    auto whole_k = kind == 0 ? w4a8::w4a8_gemv_q4k_kernel<MR, R, false> : w4a8::w4a8_gemv_q6k_kernel<MR, R, false>;
+    if (MR > 1 && kind == 0) return PB_UNSUPPORTED_SHAPE;          // not reached: two Q4_K rows run on w4a8_mma.cuh
+    auto split_k = kind == 0 ? w4a8::w4a8_gemv_q4k_kernel<1, R, true> : w4a8::w4a8_gemv_q6k_kernel<MR, R, true>;
+    auto whole_k = kind == 0 ? w4a8::w4a8_gemv_q4k_kernel<1, R, false> : w4a8::w4a8_gemv_q6k_kernel<MR, R, false>;
     // few rows: two to four warps per CTA share the rows' super-blocks (exact: the chain runs in order afterwards);
     // the most warps with which the whole grid is resident at once (a second, short wave would double the time)
     const size_t smem = (size_t)(p.K >> 8) * 4 * R * MR * sizeof(float);

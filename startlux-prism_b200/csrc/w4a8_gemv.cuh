@@ -1,7 +1,7 @@
-// W4A8 for one activation row (two against Q6_K matrices of many rows; w4a8_mma.cuh takes over from there: a layer at two rows
-// 90 -> 81 us, but 77 -> 81 at one): no tensor core - at these row counts the MMA
-// would be 3 % used and the hand-offs between its stages are what the time goes to - but integer dot products on the
-// CUDA cores, straight from the packed weights in global memory.  Same arithmetic as the other W4A8 kernels
+// W4A8 for one activation row (two against Q6_K matrices of many rows; w4a8_mma.cuh takes over from there: a layer at two
+// rows 90 -> 81 us, but 77 -> 81 at one): no tensor core - at these row counts the MMA would be 3 % used and the hand-offs
+// between its stages are what the time goes to - but integer dot products on the CUDA cores, straight from the packed
+// weights in global memory.  Same arithmetic as the other W4A8 kernels
 // (kernels/w4a8.py:14-24): exact integers inside a 256-input super-block, then per super-block, in order,
 //   Q4_K  t = d * float(acc); t = fma(-dmin, float(mins), t); y = fma(a, t, y)
 //   Q6_K  y = fma(a, d * float(acc), y)
@@ -56,9 +56,9 @@ __device__ __forceinline__ uint4 ldg_stream(const void* p) {
     return v;
 }
 
-// Sum v[0..NV) (NV = 1, 2, 4, 8 or 16) over the eight lanes that differ in bits 2, 1, 0.  While more than one value is left a
+// Sum v[0..NV) (NV = 1, 2 or 4) over the eight lanes that differ in bits 2, 1, 0.  While more than one value is left a
 // step halves them (the lane whose bit is set keeps the upper half); after that the steps are plain butterflies.  On
-// return v[0] (and v[1] for sixteen values) hold the totals of the original indices reduce8_index<NV>(lane) (+ 1).
+// return v[0] holds the total of the original index reduce8_index<NV>(lane).
 template <int NV>
 __device__ __forceinline__ void reduce8(int (&v)[NV], int lane) {
     int n = NV;
@@ -83,17 +83,15 @@ __device__ __forceinline__ void reduce8(int (&v)[NV], int lane) {
 
 template <int NV>
 __device__ __forceinline__ int reduce8_index(int lane) {
-    static_assert(NV == 1 || NV == 2 || NV == 4 || NV == 8 || NV == 16, "a power of two up to sixteen values");
+    static_assert(NV == 1 || NV == 2 || NV == 4, "a power of two up to four values");
     int base = (lane & 4) ? NV / 2 : 0;
     if (NV >= 4) base += (lane & 2) ? NV / 4 : 0;
-    if (NV >= 8) base += (lane & 1) ? NV / 8 : 0;
     return base;
 }
 
 template <int NV>
 __device__ __forceinline__ bool reduce8_owner(int lane) {
-    // with fewer than eight values the butterfly steps leave copies: the lane with the low bits clear stores
-    return NV >= 8 ? true : (lane & (8 / (NV >= 8 ? 8 : NV) - 1)) == 0;
+    return (lane & (8 / NV - 1)) == 0;             // the butterfly steps leave copies: the lane with the low bits clear stores
 }
 
 __device__ __forceinline__ int dot32(const uint4& w0, const uint4& w1, const uint4& x0, const uint4& x1) {
@@ -136,7 +134,7 @@ __device__ __forceinline__ void gemv_chain(const GemvArgs& p, const float* terms
 template <int MR, int R, bool SPLIT>
 __global__ void __launch_bounds__(SPLIT ? 128 : 32)
 w4a8_gemv_q4k_kernel(const GemvArgs p) {
-    constexpr int NV = R * MR, PD = GEMV_PD, NF = NV >= 8 ? NV / 8 : 1;   // NF: (row, activation row) pairs per lane
+    constexpr int NV = R * MR, PD = GEMV_PD;
     extern __shared__ float gemv_terms[];                          // SPLIT: [K / 256][4 * R * MR] chain terms
     const int KW = SPLIT ? (int)(blockDim.x >> 5) : 1;             // warps sharing the CTA's rows
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -146,7 +144,7 @@ w4a8_gemv_q4k_kernel(const GemvArgs p) {
     live = live < p.M ? live : p.M;
     if (live <= 0) return;
     const int NSB = p.K >> 8;
-    // the (row, activation row) pairs whose fp32 chains this lane owns: NF consecutive activation rows of one row
+    // the (row, activation row) pair whose fp32 chain this lane owns
     const int mine = reduce8_index<NV>(lane), r_o = mine / MR, m_o = mine % MR;
     const long row_o = n0 + r_o < p.N ? n0 + r_o : p.N - 1;        // rows past N read the last row and store nothing
     const uint8_t* wrow[R];
@@ -162,9 +160,8 @@ w4a8_gemv_q4k_kernel(const GemvArgs p) {
     int sc[PD][R];
     uint2 mn[PD];
     float dv[PD], dmv[PD];
-    float y[NF];
-#pragma unroll
-    for (int i = 0; i < NF; ++i) y[i] = 0.0f;
+    const int m_c = m_o < p.M ? m_o : p.M - 1;
+    float y = 0.0f;
     for (int b0 = warp; b0 < NSB; b0 += PD * KW) {
 #pragma unroll
         for (int j = 0; j < PD; ++j)
@@ -210,32 +207,24 @@ w4a8_gemv_q4k_kernel(const GemvArgs p) {
                     for (int m = 0; m < MR; ++m) v[r * MR + m] = scb[r] * dot32(lo, hi, x0[m], x1[m]);
                 }
                 reduce8<NV>(v, lane);
-#pragma unroll
-                for (int i = 0; i < NF; ++i) {                     // this lane's pairs: the same row, consecutive m
-                    const int mi = m_o + i < p.M ? m_o + i : p.M - 1;
-                    const uint4 s = __ldg((const uint4*)(p.xs + ((long)b * p.Ma + mi) * 16));
-                    const int mins = __dp4a((int)mnb.x, (int)s.x, __dp4a((int)mnb.y, (int)s.y, 0)) +
-                                     64 * __dp4a((int)mnb.x, (int)s.z, __dp4a((int)mnb.y, (int)s.w, 0));
-                    float t = __fmul_rn(dvb, __int2float_rn(v[i]));
-                    t = __fmaf_rn(ndm, __int2float_rn(mins), t);
-                    if (!SPLIT) y[i] = __fmaf_rn(__ldg(p.a + (long)b * p.Ma + mi), t, y[i]);
-                    else if (reduce8_owner<NV>(lane)) gemv_terms[b * (4 * NV) + ((lane >> 3) * R + r_o) * MR + m_o + i] = t;
-                }
+                const uint4 s = __ldg((const uint4*)(p.xs + ((long)b * p.Ma + m_c) * 16));
+                const int mins = __dp4a((int)mnb.x, (int)s.x, __dp4a((int)mnb.y, (int)s.y, 0)) +
+                                 64 * __dp4a((int)mnb.x, (int)s.z, __dp4a((int)mnb.y, (int)s.w, 0));
+                float t = __fmul_rn(dvb, __int2float_rn(v[0]));
+                t = __fmaf_rn(ndm, __int2float_rn(mins), t);
+                if (!SPLIT) y = __fmaf_rn(__ldg(p.a + (long)b * p.Ma + m_c), t, y);
+                else if (reduce8_owner<NV>(lane)) gemv_terms[b * (4 * NV) + ((lane >> 3) * R + r_o) * MR + m_o] = t;
             }
         }
     }
-    if (!SPLIT) {
-#pragma unroll
-        for (int i = 0; i < NF; ++i) gemv_store(p, y[i], n0 + r_o, m_o + i, live, reduce8_owner<NV>(lane));
-    } else {
-        gemv_chain<MR, R>(p, gemv_terms, NSB, live);
-    }
+    if (!SPLIT) gemv_store(p, y, n0 + r_o, m_o, live, reduce8_owner<NV>(lane));
+    else gemv_chain<MR, R>(p, gemv_terms, NSB, live);
 }
 
 template <int MR, int R, bool SPLIT>
 __global__ void __launch_bounds__(SPLIT ? 128 : 32)
 w4a8_gemv_q6k_kernel(const GemvArgs p) {
-    constexpr int NV = R * MR, PD = GEMV_PD, NF = NV >= 8 ? NV / 8 : 1;   // NF: (row, activation row) pairs per lane
+    constexpr int NV = R * MR, PD = GEMV_PD;
     extern __shared__ float gemv_terms[];                          // SPLIT: [K / 256][4 * R * MR] chain terms
     const int KW = SPLIT ? (int)(blockDim.x >> 5) : 1;             // warps sharing the CTA's rows
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -259,9 +248,8 @@ w4a8_gemv_q6k_kernel(const GemvArgs p) {
     uint4 ring[PD][R][2];
     short sc[PD][R];                                               // two int8 sub-block scales
     float dv[PD];
-    float y[NF];
-#pragma unroll
-    for (int i = 0; i < NF; ++i) y[i] = 0.0f;
+    const int m_c = m_o < p.M ? m_o : p.M - 1;
+    float y = 0.0f;
     for (int b0 = warp; b0 < NSB; b0 += PD * KW) {
 #pragma unroll
         for (int j = 0; j < PD; ++j)
@@ -314,22 +302,14 @@ w4a8_gemv_q6k_kernel(const GemvArgs p) {
                     }
                 }
                 reduce8<NV>(v, lane);
-#pragma unroll
-                for (int i = 0; i < NF; ++i) {
-                    const int mi = m_o + i < p.M ? m_o + i : p.M - 1;
-                    const float t = __fmul_rn(dvb, __int2float_rn(v[i]));
-                    if (!SPLIT) y[i] = __fmaf_rn(__ldg(p.a + (long)b * p.Ma + mi), t, y[i]);
-                    else if (reduce8_owner<NV>(lane)) gemv_terms[b * (4 * NV) + ((lane >> 3) * R + r_o) * MR + m_o + i] = t;
-                }
+                const float t = __fmul_rn(dvb, __int2float_rn(v[0]));
+                if (!SPLIT) y = __fmaf_rn(__ldg(p.a + (long)b * p.Ma + m_c), t, y);
+                else if (reduce8_owner<NV>(lane)) gemv_terms[b * (4 * NV) + ((lane >> 3) * R + r_o) * MR + m_o] = t;
             }
         }
     }
-    if (!SPLIT) {
-#pragma unroll
-        for (int i = 0; i < NF; ++i) gemv_store(p, y[i], n0 + r_o, m_o + i, live, reduce8_owner<NV>(lane));
-    } else {
-        gemv_chain<MR, R>(p, gemv_terms, NSB, live);
-    }
+    if (!SPLIT) gemv_store(p, y, n0 + r_o, m_o, live, reduce8_owner<NV>(lane));
+    else gemv_chain<MR, R>(p, gemv_terms, NSB, live);
 }
 
 }  // namespace w4a8

@@ -136,25 +136,24 @@ __device__ __forceinline__ void add_quad(f32x2* acc, const uint32_t (&r)[4][RW],
 
 // tm_w: weights [N, K] as {128, N, K / 128} with box {128, 128, 2}; tm_x: activations [M, K] the same way with box
 // {128, NB, 2}.  p: a_s [M, K / 32], w_s [N, K / 32], out, ldo, n_rows, M, N, K (a multiple of 128), epi (bf16, fp32 add
-// or fp32), pdl, stages.  Grid (N / 128 tiles, 1, row blocks of 2 * RW).
-template <int NB, int RW>
+// or fp32), pdl, stages.  Grid (N / 128 tiles, 1, row blocks of NB).
+template <int NB>
 __global__ void __launch_bounds__(G32<NB>::THREADS, 1)
 w8a8_g32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const SwapArgs p) {
     using C = G32<NB>;
-    constexpr int RCTA = 2 * RW;                               // activation rows this CTA owns (<= NB)
-    constexpr int RC = RW < 8 ? RW : 8;                        // rows per tensor-memory load
+    constexpr int RW = NB / 2, RC = 8;                         // activation rows per epilogue warp, per tensor-memory load
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = align1024(smem_raw);
     const int NST = p.stages;
     const int KC = p.K / BK;                                   // quads = 128-byte chunks of K
     const int QP = C::padded_quads(p.K);
-    float4* sa = (float4*)(smem + NST * C::STAGE_BYTES);       // float2 [RCTA / 2 row pairs][QP quads][4 groups]
-    Aux* aux = (Aux*)((uint8_t*)sa + C::sa_bytes(p.K, RCTA));
+    float4* sa = (float4*)(smem + NST * C::STAGE_BYTES);       // float2 [NB / 2 row pairs][QP quads][4 groups]
+    Aux* aux = (Aux*)((uint8_t*)sa + C::sa_bytes(p.K, NB));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     int live = *p.n_rows;
     live = live < p.M ? live : p.M;
-    const int n0 = blockIdx.x * BM, m0 = blockIdx.z * RCTA;
+    const int n0 = blockIdx.x * BM, m0 = blockIdx.z * NB;
     if (m0 >= live) return;                                    // whole CTA, before any barrier or allocation
     const int nst = (KC + 1) / 2;                              // stages of K this CTA walks through
     const int nslots = (KC + C::SLOT_QUADS - 1) / C::SLOT_QUADS;
@@ -283,11 +282,11 @@ w8a8_g32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
         float4 sw_ahead[C::SLOT_QUADS];
 #pragma unroll
         for (int b = 0; b < C::SLOT_QUADS; ++b) sw_ahead[b] = b < KC ? __ldg(swp + b) : make_float4(0.f, 0.f, 0.f, 0.f);
-        // the CTA's activation scales: a_s rows m0 .. m0 + RCTA - 1, one float4 per quad, read once
+        // the CTA's activation scales: a_s rows m0 .. m0 + NB - 1, one float4 per quad, read once
         {
             const int e = threadIdx.x - 32 * C::FIRST_EPI_WARP;
             float* saf = (float*)sa;
-            for (int idx = e; idx < RCTA * KC; idx += 32 * C::EPI_WARPS) {
+            for (int idx = e; idx < NB * KC; idx += 32 * C::EPI_WARPS) {
                 const int row = idx / KC, qd = idx - row * KC;
                 const int m = m0 + row;
                 const float4 v = m < live ? __ldg((const float4*)(p.a_s + (long)m * G) + qd)
