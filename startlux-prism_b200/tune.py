@@ -44,8 +44,8 @@ def graph_us(fn_of_copy, copies, iters=None, reps=5):
 
 def measure(shapes, rows, log=print, chained=True):
     """chained: rows from 2 up are timed as LinearStack launches them at few rows - every launch a programmatic
-    dependent of the one before it (pb_set_pdl) - so that the choice fits that pass; one row (the CUDA-core kernel,
-    a plain launch) is timed alone."""
+    dependent of the one before it (pb_set_pdl) - so that the choice fits that pass.  One row is timed twice: alone
+    (the CUDA-core kernel where that takes the call) and, under "1p", chained on the tensor-core kernel."""
     import torch
 
     from . import _lib, quant, w8a8
@@ -59,7 +59,9 @@ def measure(shapes, rows, log=print, chained=True):
         for residual in (False, True):
             key = f"{N}x{K}" + ("r" if residual else "")
             table[key] = {}
-            for M in rows:
+            for row in [r for m in rows for r in ([m, "1p"] if m == 1 and chained else [m])]:
+                M = 1 if row == "1p" else row
+                chain = chained and row != 1
                 a = torch.randint(-127, 128, (M, K), dtype=torch.int8, device=dev, generator=gen)
                 sa = torch.rand(M, device=dev, generator=gen) * 1e-2
                 nr = torch.tensor([M], dtype=torch.int32, device=dev)
@@ -74,10 +76,10 @@ def measure(shapes, rows, log=print, chained=True):
 
                         def call(c):
                             pend[0] = w8a8.gemm(a, sa, ws[c], sw, out, nr, K, epi=int(residual), cfg=split,
-                                                slots=slots if defer else None)
-                            if chained and M > 1 and pend[0] is not None:
+                                                slots=slots if defer else None, pdl=chain)
+                            if chain and pend[0] is not None:
                                 quant.fold(out, slots, pend[0], nr, M)        # the fold is part of the chain
-                        if chained and M > 1:
+                        if chain:
                             before = _lib.lib().pb_set_pdl(1)
                             try:
                                 us = graph_us(call, copies)
@@ -89,15 +91,16 @@ def measure(shapes, rows, log=print, chained=True):
                                 us += graph_us(lambda c: quant.fold(out, slots, pend[0], nr, M), 1, iters=8)
                         if best is None or us < best["us"]:
                             best = {"split": split, "defer": bool(defer), "us": round(us, 2)}
-                table[key][str(M)] = best
-                log(f"{key} M={M}: {best}")
+                table[key][str(row)] = best
+                log(f"{key} M={row}: {best}")
         del ws
         torch.cuda.empty_cache()
     return table
 
 
 def load_table(path=None):
-    """{(N, K, residual): {M: {"split", "defer", "us"}}} from the table file, or {} when there is none."""
+    """{(N, K, residual): {M: {"split", "defer", "us"}}} from the table file, or {} when there is none.  M: a row count, or
+    "1p" (one row as a programmatic dependent on the tensor-core kernel)."""
     path = path or os.environ.get("PRISM_B200_GEMM_TABLE") or TABLE
     if not os.path.exists(path):
         return {}
@@ -105,7 +108,7 @@ def load_table(path=None):
     out = {}
     for key, by_m in raw.items():
         n, k = key.rstrip("r").split("x")
-        out[(int(n), int(k), key.endswith("r"))] = {int(m): v for m, v in by_m.items()}
+        out[(int(n), int(k), key.endswith("r"))] = {m if m == "1p" else int(m): v for m, v in by_m.items()}
     return out
 
 
@@ -122,7 +125,7 @@ def main(argv=None):
     table = measure(shapes, rows, chained=not args.plain)
     doc = {"gpu": torch.cuda.get_device_name(0), "sms": torch.cuda.get_device_properties(0).multi_processor_count,
            "method": "CUDA graph of calls over rotating weight copies (> 3 x L2), best of 5 replays"
-           + ("" if args.plain else "; 2 rows and up as a chain of programmatic dependent launches"), "table": table}
+           + ("" if args.plain else "; 2 rows and up, and 1p, as a chain of programmatic dependent launches"), "table": table}
     with open(args.out, "w") as f:
         json.dump(doc, f, indent=1)
     print(f"wrote {args.out}")

@@ -14,6 +14,7 @@ Kernel choice (this module's table replaces the reference's per-GPU JSON tables)
 128 x 256 tile kernel; up to 64 rows -> the operand-swapped split-K kernel, the splits' int32 sums either deferred to
 the caller's `slots` (epi 1) or added inside the kernel through a workspace.
 """
+import math
 import weakref
 from typing import NamedTuple
 
@@ -129,10 +130,11 @@ def _choice(M, N, K, residual, chained=False):
     by_m = _TABLE.get((N, K, bool(residual)))
     if not by_m:
         return None
-    import math
     # the one-row entry was measured on the CUDA-core kernel: it says nothing about the tensor-core kernel, which runs at
-    # two rows up and in a chain of programmatic dependents of one row
-    rows = [x for x in by_m if x > GEMV_ROWS] if M > GEMV_ROWS or chained else list(by_m)
+    # two rows up and in a chain of programmatic dependents of one row (an entry "1p" of its own, where it was measured)
+    if chained and M <= GEMV_ROWS and "1p" in by_m:
+        return by_m["1p"]
+    rows = [x for x in by_m if x != "1p" and (x > GEMV_ROWS or (M <= GEMV_ROWS and not chained))]
     if not rows:
         return None
     m = min(rows, key=lambda x: abs(math.log(x) - math.log(max(M, 1))))

@@ -53,6 +53,21 @@ def test_pdl_switch_belongs_to_its_thread(lib):
     assert lib.pb_set_pdl(0) == 0
 
 
+def test_one_row_chain_takes_its_own_table_entry(monkeypatch, tmp_path):
+    """A chained one-row product uses the entry that was measured for it, the next larger row count when there is none, and
+    never the CUDA-core kernel's; nothing else sees the chained entry."""
+    import json
+
+    from prism_b200 import tune
+    e = {m: {"split": i + 1, "defer": False, "us": 1.0} for i, m in enumerate(("1", "8", "64", "1p"))}
+    path = tmp_path / "table.json"
+    path.write_text(json.dumps({"table": {"256x512": e, "256x1024": {m: e[m] for m in ("1", "8", "64")}}}))
+    monkeypatch.setattr(w8a8, "_TABLE", tune.load_table(str(path)))
+    split = lambda M, K, chained: w8a8._choice(M, 256, K, False, chained)["split"]          # noqa: E731
+    assert (split(1, 512, False), split(1, 512, True), split(1, 1024, True)) == (1, 4, 2)
+    assert (split(2, 512, False), split(2, 512, True), split(60, 512, True)) == (2, 2, 3)
+
+
 class _Recorder:
     """The library with every launch replaced by a note of its arguments."""
 
