@@ -11,13 +11,14 @@
 // The super-block's term t_b = d * float(acc) [- dmin * float(mins)] goes to shared memory; the CTA's WK warp groups
 // work on WK consecutive super-blocks, and the threads then run the chain y = fma(a_b, t_b, y) over them in order,
 // one round later (two term buffers, one barrier per round).  So K is split over warps without a change of bits, and
-// a 5120-row projection still fills the SMs with CTAs of 32 rows.
+// a 5120-row Q4_K projection is 320 CTAs of 16 rows (Q6_K: 80 to 160 of 64 or 32).
 // Operands come through a ring of ST rounds by cp.async (16 bytes a lane, rows of 128 bytes whole), XOR-swizzled so
 // that every ldmatrix is free of bank conflicts; the WN warps of a super-block share its activations.
 //
-// What bounds it: instruction issue (ncu, 16 rows x 34816 x 5120: 2.4 instructions a clock and SM, DRAM a third busy): per
-// 16 x 256 weights about 400 warp instructions, of which unpacking, IMADs and MMAs are 130 at 16 rows.  Measured, one
-// launch with weights from HBM, before (tcgen05 with the sums through tensor memory; dp4a up to eight rows) and after:
+// What bounds it: instruction issue, with too few warps to fill the slots (ncu, Q4_K at 12 rows: 34816 x 5120 54 % of them, DRAM
+// 45 %, two CTAs of four warps per SM, fixed latencies the first stall; 6144 x 5120 45 %, the ring's copies the first stall).
+// Measured, one launch with weights from HBM, before (tcgen05 with the sums through tensor memory; dp4a up to eight rows)
+// and after:
 //   Q4_K  6144 x 5120   8 rows 18.2 ->  7.1 us   12 rows 17.2 ->  9.1    32 rows 21.9 -> 15.4
 //         34816 x 5120  8 rows 37.3 -> 21.4      12 rows 42.4 -> 27.6    32 rows 81.6 -> 46.4
 //   Q6_K  5120 x 17408  8 rows 45.0 -> 24.0      12 rows 72.5 -> 33.5    32 rows 142.5 -> 56.9

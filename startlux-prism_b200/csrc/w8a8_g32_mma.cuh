@@ -10,8 +10,9 @@
 // against 8 of the tensor pipe.  A warp takes 16 * NT weight rows x 8 * MT activation rows over the whole of K (the chain is
 // serial), a CTA WN x WM such warps on one ring of ST stages of KQ * 128 bytes of K, filled by cp.async and XOR-swizzled for
 // ldmatrix; the activation scales are staged as row pairs, so that one 16-byte read serves two groups of NT tiles.
-// What bounds it: at NT = 1 shared-memory reads (ncu: 67 % of its wavefronts, its latency the first stall), at NT = 2 these
-// and the fp32 pipe alike; below 17 rows the latency of one warp per scheduler walking the chain.
+// What bounds it: at NT = 1 with many rows shared-memory reads (ncu of a first version: 67 % of the wavefronts), hence NT = 2; there
+// the chain's fp32 pipe at many rows (500 rows: 55 % busy, issue slots 52 %, shared memory 49 %), at 48 rows the latencies of
+// the chain with two warps per scheduler (fp32 pipe 41 %, DRAM 34 %), and below 17 rows those of one warp per scheduler.
 // Measured against the tcgen05 kernel that ran all of these before (us, one launch):
 //   5120 x 5120   8 rows 12.8 -> 11.0   16 rows 14.6 -> 12.5   64 rows 29.5 -> 25.6   256 rows 84.6 -> 56.6
 //   7168 x 5120   500 rows 189 -> 141   1000 rows 337 -> 258;   34816 x 5120   256 rows 421 -> 317
