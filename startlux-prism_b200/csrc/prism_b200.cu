@@ -1594,9 +1594,13 @@ int pb_mxfp4_prepare_sf(const void* s, void* dst, int rows, int K, void* stream)
 int pb_mxfp4_quant(const void* x, int x_fp32, const float* inv, void* q, void* s, int n, int K, void* stream) {
     if (!x || !q || !s || n <= 0 || K <= 0) return PB_BAD_ARGUMENT;
     if (K % 32 || !aligned16(x) || ((uintptr_t)q & 3)) return PB_UNSUPPORTED_SHAPE;
-    dim3 grid((K / 8 + 255) / 256, n);
-    if (x_fp32) mxfp4::mxfp4_quant_kernel<false><<<grid, 256, 0, (cudaStream_t)stream>>>(x, inv, (uint8_t*)q, (uint8_t*)s, n, K);
-    else mxfp4::mxfp4_quant_kernel<true><<<grid, 256, 0, (cudaStream_t)stream>>>(x, inv, (uint8_t*)q, (uint8_t*)s, n, K);
+    const long vecs = (long)n * (K / 8);
+    // four vectors a thread where that still gives every SM several CTAs
+    const int u = vecs >= (long)sm_count() * 256 * 16 ? 4 : 1;
+    const unsigned grid = (unsigned)((vecs + 256 * u - 1) / (256 * u));
+    auto kern = x_fp32 ? (u == 4 ? mxfp4::mxfp4_quant_kernel<false, 4> : mxfp4::mxfp4_quant_kernel<false, 1>)
+                       : (u == 4 ? mxfp4::mxfp4_quant_kernel<true, 4> : mxfp4::mxfp4_quant_kernel<true, 1>);
+    kern<<<grid, 256, 0, (cudaStream_t)stream>>>(x, inv, (uint8_t*)q, (uint8_t*)s, vecs, K / 8);
     PB_CUDA(cudaGetLastError());
     return PB_OK;
 }

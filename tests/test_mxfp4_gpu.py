@@ -48,6 +48,45 @@ def test_quantize_act_oracle(dev, n, k):
     assert rel < 0.2                                      # tests/test_mxfp4.py:41-51
 
 
+def quant_by_thresholds(x, inv):
+    """The quantizer's definition in numpy: a block's exponent from its largest magnitude (a NaN does not count), magnitude codes by
+    strict thresholds, the sign bit where v < 0."""
+    v = x * inv if inv is not None else x
+    b = v.reshape(x.shape[0], -1, 32)
+    amax = np.maximum(np.where(np.isnan(b), 0, np.abs(b)).max(2), np.float32(1e-30)).astype(np.float32)
+    bits = amax.view(np.uint32)
+    e = np.clip((bits >> 23).astype(np.int32) - np.where((bits & 0x7fffff) <= 0x400000, 129, 128), -127, 127)
+    with np.errstate(all="ignore"):
+        a = np.abs(b) * np.ldexp(np.float32(1), -e).astype(np.float32)[..., None]
+        c = sum((a > t).astype(np.uint8) for t in (0.25, 0.75, 1.25, 1.75, 2.5, 3.5, 5.0)) | np.where(b < 0, 8, 0).astype(np.uint8)
+    c = c.reshape(x.shape)
+    return c[:, ::2] | (c[:, 1::2] << 4), (e + 127).astype(np.uint8)
+
+
+@pytest.mark.parametrize("n", [3, 601])                   # one vector a thread, four vectors a thread
+@pytest.mark.parametrize("kind", ["bf16", "f32", "scaled"])
+def test_quantize_act_edges(dev, n, kind):
+    """Halfway values and their neighbours on both sides, both zeros, values far below the block's largest, infinities and
+    NaN, in every block position."""
+    k = 8192
+    g = np.random.default_rng(n)
+    half = np.array([0.25, 0.75, 1.25, 1.75, 2.5, 3.5, 5.0, 6.0, 0.5, 1.0, 3.0, 0.0, -0.0, 1e-38, 2.0 ** -140], np.float32)
+    near = np.concatenate([half, np.nextafter(half, np.float32(9)), np.nextafter(half, np.float32(-9))])
+    near = np.concatenate([near, half * np.float32(1 + 2.0 ** -7), half * np.float32(1 - 2.0 ** -8)])
+    v = g.choice(np.concatenate([near, -near]).astype(np.float32), (n, k // 32, 32))
+    v[:, :, 0] = 6.0                                      # the block's scale is 2^e
+    v = v * np.ldexp(np.float32(1), g.integers(-40, 40, (n, k // 32, 1))).astype(np.float32)
+    v[g.random(v.shape) < 2e-4] = np.nan
+    v[g.random(v.shape) < 1e-4] = np.inf
+    v[g.random(v.shape) < 1e-4] = -np.inf
+    v = torch.from_numpy(g.permuted(v, axis=2).reshape(n, k))
+    inv = torch.from_numpy(g.choice(np.array([1, 0.5, 1.1, 3], np.float32), k)) if kind == "scaled" else None
+    x = v if kind == "f32" else v.bfloat16()
+    q, s = quant_gpu(x, dev, inv)
+    rq, rs = quant_by_thresholds(x.float().numpy(), None if inv is None else inv.numpy())
+    assert same(s, rs) and same(q, rq)
+
+
 def rel_fro(got, ref):
     return float(np.linalg.norm(got.astype(np.float64) - ref) / np.linalg.norm(ref))
 
