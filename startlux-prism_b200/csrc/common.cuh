@@ -75,6 +75,16 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
+// Has the phase with `parity` completed?  Never waits (try_wait may).
+__device__ __forceinline__ bool mbar_peek(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
 // The same test, but the thread may stay suspended up to `ns` nanoseconds while the phase is incomplete (it is woken
 // when the phase completes): a waiting warp then issues next to nothing instead of spinning against the working ones.
 __device__ __forceinline__ bool mbar_test_sleep(uint32_t bar, uint32_t parity, uint32_t ns) {

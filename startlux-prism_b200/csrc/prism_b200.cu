@@ -22,6 +22,7 @@
 #include "w4a8_mma.cuh"
 #include "w8a8_gemv.cuh"
 #include "mxfp4_gemm.cuh"
+#include "mxfp4_few.cuh"
 #include "mxfp4_gemv.cuh"
 
 namespace {
@@ -662,6 +663,16 @@ int launch_w4a8_few(const w4a8::GemvArgs& p, cudaStream_t st) {
         return p.M <= 16 ? launch_w4a8_mma<KIND, 1, 1, 1, 4, 4>(p, st) : launch_w4a8_mma<KIND, 2, 1, 1, 4, 3>(p, st);
     if (p.M <= 8) return launch_w4a8_mma<KIND, 1, 1, 2, 4, 2>(p, st);
     return p.M <= 16 ? launch_w4a8_mma<KIND, 2, 2, 2, 4, 2>(p, st) : launch_w4a8_mma<KIND, 4, 1, 4, 2, 2>(p, st);
+}
+
+template <int ST>
+int launch_mxfp4_few(const CUtensorMap& tw, const CUtensorMap& tx, const mxfp4::FewArgs& p, int grid, cudaStream_t st) {
+    auto kern = mxfp4::mxfp4_few_kernel<ST>;
+    int rc;
+    if ((rc = set_smem(kern, mxfp4::few_smem<ST>()))) return rc;
+    kern<<<grid, 224, mxfp4::few_smem<ST>(), st>>>(tw, tx, p);
+    PB_CUDA(cudaGetLastError());
+    return PB_OK;
 }
 
 // One activation row (two for Q6_K): integer dot products on the CUDA cores (w4a8_gemv.cuh).
@@ -1618,6 +1629,25 @@ long pb_mxfp4_workspace_bytes(int M, int N, int split) {
 int pb_mxfp4_counters(int M, int N) {
     if (M <= 0 || N <= 0) return 0;
     return ((M + 127) / 128) * ((N + 127) / 128);
+}
+
+int pb_mxfp4_gemm_few(const void* aq, const void* a_s, const void* bq, const void* b_sf, void* out, long ldo, int M, int N, int K,
+                      int epi, void* stream) {
+    if (!aq || !a_s || !bq || !b_sf || !out || M <= 0 || N <= 0 || K <= 0 || ldo < N) return PB_BAD_ARGUMENT;
+    if (epi != 0 && epi != 1) return PB_BAD_ARGUMENT;
+    if (K % 256 || M > mxfp4::FEW_ROWS) return PB_UNSUPPORTED_SHAPE;
+    if (!aligned16(aq) || !aligned16(bq) || !aligned16(b_sf) || ((uintptr_t)a_s & 3)) return PB_BAD_ARGUMENT;
+    const int tiles = (N + 127) / 128, cols = (M + 15) & ~15;
+    int parts = 1;
+    while (parts < 4 && tiles * parts * 2 <= sm_count()) parts *= 2;
+    CUtensorMap tw, tx;
+    int rc;
+    if ((rc = tensor_map(&tw, bq, K / 2, N, K / 2, 128, 128 / parts, 0))) return rc;
+    if ((rc = tensor_map(&tx, aq, K / 2, M, K / 2, 128, cols, 0))) return rc;
+    const mxfp4::FewArgs p{(const uint8_t*)a_s, (const uint8_t*)b_sf, out, ldo, M, N, K, epi, cols, parts};
+    // one CTA per SM takes all of its shared memory as stages, more than that share it
+    if (tiles * parts <= sm_count()) return launch_mxfp4_few<8>(tw, tx, p, tiles * parts, (cudaStream_t)stream);
+    return launch_mxfp4_few<4>(tw, tx, p, tiles * parts, (cudaStream_t)stream);
 }
 
 int pb_mxfp4_gemm_split(const void* aq, const void* a_sf, const void* bq, const void* b_sf, void* out, long ldo, int M,

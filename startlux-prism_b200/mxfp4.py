@@ -132,6 +132,9 @@ def prepare(w: MX4) -> MX4:
 cutlass_prepare = prepare       # the reference's name for the same step (kernels/mxfp4.py:214)
 
 
+FEW_ROWS = 64                   # rows up to which gemm runs mxfp4_few_kernel
+
+
 def _sm_count():
     from .w8a8 import SM_COUNT
     return SM_COUNT
@@ -185,6 +188,15 @@ def gemm(a_q, a_s, w: MX4, out, n_rows, epi=0, out_stride=None, split=None):
         # one row against a matrix of few rows: the CUDA-core kernel (measured: level with the tensor-core kernel on a
         # 34816-row matrix and behind it from two rows, where its decode arithmetic is the bound)
         return gemv(a_q, a_s, w, out, M, epi, out_stride)
+    ldo = out.stride(0) if out_stride is None else out_stride
+    split = 1 if split is None else pick_split(M, N, K) if split == "auto" else max(1, int(split))
+    if split == 1 and M <= FEW_ROWS and K % 256 == 0 and a_s.data_ptr() % 4 == 0:
+        # a decode batch: the kernel that reads the scales as the quantizer wrote them (same bits)
+        rc = _lib.lib().pb_mxfp4_gemm_few(_lib.ptr(a_q), _lib.ptr(a_s), _lib.ptr(w.q), _lib.ptr(w.cs), _lib.ptr(out), ldo, M, N, K,
+                                          epi, _lib.stream())
+        if rc:
+            _lib.check(rc, f"mxfp4 gemm M={M} N={N} K={K} epi={epi}")
+        return
     key = (a_q.shape[0], K, a_q.device.index)
     need = _lib.lib().pb_mxfp4_sf_bytes(a_q.shape[0], K)
     sfa = _ACT_SF.get(key)
@@ -194,8 +206,6 @@ def gemm(a_q, a_s, w: MX4, out, n_rows, epi=0, out_stride=None, split=None):
         sfa = _ACT_SF[key] = torch.zeros(need, dtype=torch.uint8, device=a_q.device)
     L = _lib.lib()
     _lib.check(L.pb_mxfp4_prepare_sf(_lib.ptr(a_s), _lib.ptr(sfa), a_q.shape[0], K, _lib.stream()), "mxfp4 prepare_sf")
-    ldo = out.stride(0) if out_stride is None else out_stride
-    split = 1 if split is None else pick_split(M, N, K) if split == "auto" else max(1, int(split))
     ws = counters = None
     if split > 1:
         from . import w8a8 as KW

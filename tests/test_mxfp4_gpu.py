@@ -223,3 +223,28 @@ def test_wide_tiles_same_bits(dev):
         small = torch.zeros(64, N, dtype=torch.bfloat16, device=dev)
         mxfp4.gemm(q[r0:r0 + 64].contiguous(), s[r0:r0 + 64].contiguous(), wd, small, 64)
         assert same(big[r0:r0 + 64].contiguous(), small)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 40, 256), (15, 1000, 2304), (16, 132, 8704), (17, 9500, 512), (33, 4800, 1280), (48, 20000, 768),
+                                   (63, 2500, 4352), (64, 19072, 256)])
+def test_few_rows(dev, M, N, K):
+    """The decode kernel: row counts around its steps of 16, weight tiles whole, halved and quartered over CTAs and ending inside a
+    part, K shorter and longer than its stages, out a column slice.  The bits of the many-rows kernel."""
+    g = torch.Generator().manual_seed(M + N)
+    w = mxfp4.MX4(torch.randint(0, 256, (N, K // 2), generator=g, dtype=torch.uint8).to(dev),
+                  torch.randint(110, 124, (N, K // 32), generator=g, dtype=torch.uint8).to(dev), N, K)
+    wd = mxfp4.prepare(w)
+    q, s = quant_gpu(synth.activations(M + 65, K, seed=M + 7), dev)
+    want = torch.zeros(M + 65, N, dtype=torch.bfloat16, device=dev)
+    mxfp4.gemm(q, s, wd, want, M + 65)
+    h0 = torch.randn(M + 2, N + 4, generator=g).to(dev)
+    h, ref = h0.clone(), torch.zeros(M + 65, N, device=dev)
+    ref[:M] = h0[:M, 1:1 + N]
+    mxfp4.gemm(q, s, wd, ref, M + 65, epi=1)
+    out = torch.full((M + 2, N + 4), 3.0, dtype=torch.bfloat16, device=dev)
+    mxfp4.gemm(q[:M], s[:M], wd, out[:M, 3:3 + N], M)
+    mxfp4.gemm(q[:M], s[:M], wd, h[:M, 1:1 + N], M, epi=1)
+    assert same(out[:M, 3:3 + N].contiguous(), want[:M].contiguous())
+    assert same(h[:M, 1:1 + N].contiguous(), ref[:M].contiguous())
+    assert bool((out[M:] == 3).all()) and bool((out[:, :3] == 3).all()) and bool((out[:, 3 + N:] == 3).all())
+    assert same(h[M:], h0[M:]) and same(h[:, :1], h0[:, :1]) and same(h[:, 1 + N:], h0[:, 1 + N:])
