@@ -293,7 +293,7 @@ mxfp4_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0, buf = 0, sfp = 0;
             uint32_t phase = 0, bphase = 0;
             bool ok = true;
@@ -586,7 +586,7 @@ mxfp4_gemm256_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // MMA issuer.  The scale factors' copies into tensor memory are another thread's (warp 2): one thread doing
             // both issued twelve asynchronous instructions per K block, about 700 cycles against 570 of MMA time.
             int stage = 0;
@@ -627,7 +627,7 @@ mxfp4_gemm256_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
             }
         }
     } else if (warp == 2) {
-        if (lane == 0) {
+        if (elect_one()) {
             // Scale factors: shared memory -> tensor memory (two alternating sets), one K block ahead of its MMAs.  A
             // set is rewritten only after the MMAs of the K block two before have completed (that block's `empty`).
             int stage = 0;

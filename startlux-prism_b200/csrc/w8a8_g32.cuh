@@ -228,7 +228,7 @@ w8a8_g32_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
             }
         }
     } else if (warp < C::FIRST_EPI_WARP) {
-        if (lane == 0) {
+        if (elect_one()) {
             // Stage i belongs to issuing thread i % 2: a thread's loop iteration (two barrier waits, eight MMAs, two
             // commits) takes about 1,500 cycles, twice what the tensor core needs for the stage.  An accumulator slot
             // is two consecutive stages, one of each thread (16 rows), or one stage (32 rows); every stage's thread

@@ -596,7 +596,7 @@ w8a8_tile_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer (one thread)
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = umma_idesc_i8(BM, BN);
             int stage = 0, buf = 0;
             uint32_t phase = 0, bphase = 0;
@@ -604,7 +604,7 @@ w8a8_tile_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             // An mbarrier test costs this thread about 200 cycles before its answer can be used, as much as issuing
             // two MMAs.  So the test of the NEXT stage's barrier is issued before the current stage's MMAs and its
             // answer read after them: the thread stays ahead of the tensor core (512 cycles per stage).
-            bool ready = mbar_test(smem_u32(&aux->full[0]), 0);
+            bool ready = mbar_peek(smem_u32(&aux->full[0]), 0);
             for (int u = blockIdx.x; u < num_units && ok; u += gridDim.x) {
                 const Unit un = unit_of(u, full, split, kb_per_split, KB);
                 const int kb_begin = un.kb0, kb_end = un.kb1;
@@ -618,7 +618,7 @@ w8a8_tile_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     }
                     const int nstage = stage + 1 == C::STAGES ? 0 : stage + 1;
                     const uint32_t nphase = nstage == 0 ? phase ^ 1 : phase;
-                    const bool ready_next = mbar_test(smem_u32(&aux->full[nstage]), nphase);
+                    const bool ready_next = mbar_peek(smem_u32(&aux->full[nstage]), nphase);
                     tc_fence_after();
                     uint8_t* st = smem + stage * C::STAGE_BYTES;
                     const uint64_t ad = umma_desc_k128(smem_u32(st));
@@ -844,7 +844,7 @@ w8a8_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer (the leader's one thread)
-        if (leader && lane == 0) {
+        if (leader && elect_one()) {
             const uint32_t idesc = umma_idesc_i8(2 * BM, BN);
             int stage = 0, buf = 0;
             uint32_t phase = 0, bphase = 0;
@@ -1171,7 +1171,7 @@ w8a8_swap_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             if (!ok) drain_armed(aux, NST, armed_parity, armed_mask);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = umma_idesc_i8(BM, NB);
             int stage = 0, ring = 0;
             uint32_t phase = 0, rphase = 0;
@@ -1193,7 +1193,7 @@ w8a8_swap_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
                 }
                 const int nstage = stage + 1 == NST ? 0 : stage + 1;
                 const uint32_t nphase = nstage == 0 ? phase ^ 1 : phase;
-                const bool ready_next = mbar_test(smem_u32(&aux->full[nstage]), nphase);
+                const bool ready_next = mbar_peek(smem_u32(&aux->full[nstage]), nphase);
                 tc_fence_after();
                 uint8_t* st = smem + stage * C::STAGE_BYTES;
                 const uint64_t ad = umma_desc_k128(smem_u32(st));

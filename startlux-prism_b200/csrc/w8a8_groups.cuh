@@ -96,7 +96,7 @@ w8a8_groups_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             if (!ok) drain_armed(aux, C::STAGES, armed_parity, armed_mask);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = umma_idesc_i8(BM, NB);
             int stage = 0, ring = 0, in_group = 0;
             uint32_t phase = 0, rphase = 0;
