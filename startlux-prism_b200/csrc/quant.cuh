@@ -480,14 +480,22 @@ __device__ __forceinline__ void store_g_warp(const float (&v)[8], int8_t* __rest
     for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
     amax = warp_max(amax);
     const float scale = __fdiv_rn(fmaxf(amax, 1e-10f), 127.0f);
-    int qi[8], S = 0;
+    // the values as quant8 rounds them (an IEEE division each was most of the kernel's instructions); a NaN or an infinity among them
+    // takes the divisions, whose conversion makes a NaN 0
+    float z = 0.0f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        qi[j] = __float2int_rn(__fdiv_rn(v[j], scale));
-        S += qi[j];
+    for (int j = 0; j < 8; ++j) z = __fmaf_rn(v[j], 0.0f, z);
+    uint2 w;
+    if (z != z) {
+        int qi[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) qi[j] = __float2int_rn(__fdiv_rn(v[j], scale));
+        w = make_uint2(pack4(qi[0], qi[1], qi[2], qi[3]), pack4(qi[4], qi[5], qi[6], qi[7]));
+    } else {
+        w = quant8<false>(v, scale, __fdiv_rn(1.0f, scale));
     }
-    *(uint2*)(q + t * K + (long)b * 256 + lane * 8) =
-        make_uint2(pack4(qi[0], qi[1], qi[2], qi[3]), pack4(qi[4], qi[5], qi[6], qi[7]));
+    *(uint2*)(q + t * K + (long)b * 256 + lane * 8) = w;
+    int S = __dp4a((int)w.x, 0x01010101, __dp4a((int)w.y, 0x01010101, 0));
     S += __shfl_xor_sync(0xffffffffu, S, 1);
     S += __shfl_xor_sync(0xffffffffu, S, 2);
     if (lane == 0) a[(long)b * Ma + t] = scale;

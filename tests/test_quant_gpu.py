@@ -71,6 +71,27 @@ def test_rows_g(dev, T, K, live):
     assert same(q, rq) and same(a, ra) and same(xs, rxs)
 
 
+def test_rows_g_special_values(dev):
+    """NaN, infinities and values halfway between two steps: numpy's rounded IEEE quotients, 0 where the quotient is NaN (the
+    maximum does not count a NaN)."""
+    T, K = 5, 4096
+    g = np.random.default_rng(1)
+    v = (g.integers(-254, 255, (T, K)) * np.float32(0.5)).astype(np.float32)      # with 127 in every block: halves are exact
+    v[:, ::256] = 127.0
+    v[g.random(v.shape) < 1e-3] = np.nan
+    v[3, 300], v[4, 700], v[4, 701] = np.inf, -np.inf, np.nan
+    b = v.reshape(T, K // 256, 256)
+    with np.errstate(all="ignore"):
+        scale = (np.where(np.isnan(b), 0, np.abs(b)).max(2).clip(1e-10) / np.float32(127)).astype(np.float32)
+        want = np.nan_to_num(np.rint(b / scale[..., None]), nan=0.0).astype(np.int8).reshape(T, K)
+    q = torch.empty(T, K, dtype=torch.int8, device=dev)
+    a, xs = torch.empty(K // 256, T, device=dev), torch.empty(K // 256, T, 16, dtype=torch.int8, device=dev)
+    quant.rows_g(torch.from_numpy(v).to(dev), q, a, xs, n_rows(T, dev), T)
+    assert same(q, want) and same(a, np.ascontiguousarray(scale.T))
+    S = want.reshape(T, K // 256, 8, 32).astype(np.int32).sum(3).transpose(1, 0, 2)
+    assert same(xs, np.concatenate([S & 63, S >> 6], 2).astype(np.int8))
+
+
 @pytest.mark.parametrize("T,FF,live", [(5, 17408, 5), (3, 1024, 2), (2, 4352, 2)])
 def test_swiglu_q8(dev, T, FF, live):
     g = torch.Generator().manual_seed(FF)
