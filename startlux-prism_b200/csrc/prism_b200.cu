@@ -784,55 +784,57 @@ bool w4a8_no_gemv() {
 }
 
 // Row-pipelined quantizers (quant_pipe.cuh): persistent CTAs, rows staged in shared memory by bulk copies.
-template <int KIND, int VPT, bool BF16>
+template <int KIND, int VPT, bool BF16, int MAXT, int MINB, int G>
 int launch_pipe_v(bool full, const quant::PipeArgs& p, int grid, int threads, int smem, cudaStream_t st) {
     int rc;
-    if (full) {
-        auto k = quant::row_pipe_kernel<KIND, VPT, BF16, true, 576>;
-        if ((rc = set_smem(k, 200 * 1024))) return rc;
-        k<<<grid, threads, smem, st>>>(p);
-    } else {
-        auto k = quant::row_pipe_kernel<KIND, VPT, BF16, false, 576>;
-        if ((rc = set_smem(k, 200 * 1024))) return rc;
-        k<<<grid, threads, smem, st>>>(p);
-    }
+    auto k = full ? quant::row_pipe_kernel<KIND, VPT, BF16, true, MAXT, MINB, G> : quant::row_pipe_kernel<KIND, VPT, BF16, false, MAXT, MINB, G>;
+    if ((rc = set_smem(k, 220 * 1024))) return rc;
+    k<<<grid, threads, smem, st>>>(p);
+    PB_CUDA(cudaGetLastError());
     return PB_OK;
 }
 
 template <int KIND, bool BF16>
 int launch_pipe(bool full, quant::PipeArgs p, cudaStream_t st) {
-    const int nvec = p.K / 8;
+    const int nvec = p.K / 8, sms = sm_count();
+    const auto threads_for = [&](int vpt) { return ((nvec + vpt - 1) / vpt + 31) / 32 * 32; };
+    if constexpr (KIND == quant::PIPE_ROWS) if (nvec <= 640) {
+        // short rows: four CTAs per SM, 50 KB of row ring each
+        const int stages = (50 * 1024) / p.row_bytes;
+        p.stages = stages > 8 ? 8 : stages;
+        const int grid = p.T < 4 * sms ? p.T : 4 * sms, smem = p.stages * p.row_bytes + 128;
+        if (nvec <= 320) return launch_pipe_v<KIND, 1, BF16, 320, 4, 1>(full, p, grid, threads_for(1), smem, st);
+        return launch_pipe_v<KIND, 2, BF16, 320, 4, 1>(full, p, grid, threads_for(2), smem, st);
+    }
     // two CTAs per SM: about 100 KB of row ring each
     int stages = (100 * 1024) / p.row_bytes;
     int per_sm = 2;
     if (stages < 2) {                                             // very long rows: one CTA per SM
-        stages = (199 * 1024) / p.row_bytes;
+        stages = (216 * 1024) / p.row_bytes;
         per_sm = 1;
     }
     if (stages < 2) return PB_UNSUPPORTED_SHAPE;
     if (stages > 8) stages = 8;
     p.stages = stages;
     const int smem = stages * p.row_bytes + 128;
-    int grid = sm_count() * per_sm;
+    int grid = sms * per_sm;
     if (grid > p.T) grid = p.T;
+    if constexpr (KIND == quant::PIPE_SWIGLU)
+        if (per_sm == 1 && stages >= 3 && nvec <= 5 * 448)
+            return launch_pipe_v<KIND, 5, BF16, 896, 1, 2>(full, p, grid, 2 * threads_for(5), smem, st);
     // vectors of 8 inputs per thread, then just enough threads (whole warps) to cover the row
-    const int vpt = (nvec + 575) / 576;
-    const int threads = ((nvec + vpt - 1) / vpt + 31) / 32 * 32;
-    int rc;
+    const int vpt = (nvec + 575) / 576, threads = threads_for(vpt);
     switch (vpt) {
-        case 1: rc = launch_pipe_v<KIND, 1, BF16>(full, p, grid, threads, smem, st); break;
-        case 2: rc = launch_pipe_v<KIND, 2, BF16>(full, p, grid, threads, smem, st); break;
-        case 3: rc = launch_pipe_v<KIND, 3, BF16>(full, p, grid, threads, smem, st); break;
-        case 4: rc = launch_pipe_v<KIND, 4, BF16>(full, p, grid, threads, smem, st); break;
-        case 5: rc = launch_pipe_v<KIND, 5, BF16>(full, p, grid, threads, smem, st); break;
-        case 6: rc = launch_pipe_v<KIND, 6, BF16>(full, p, grid, threads, smem, st); break;
-        case 7: rc = launch_pipe_v<KIND, 7, BF16>(full, p, grid, threads, smem, st); break;
-        case 8: rc = launch_pipe_v<KIND, 8, BF16>(full, p, grid, threads, smem, st); break;
+        case 1: return launch_pipe_v<KIND, 1, BF16, 576, 1, 1>(full, p, grid, threads, smem, st);
+        case 2: return launch_pipe_v<KIND, 2, BF16, 576, 1, 1>(full, p, grid, threads, smem, st);
+        case 3: return launch_pipe_v<KIND, 3, BF16, 576, 1, 1>(full, p, grid, threads, smem, st);
+        case 4: return launch_pipe_v<KIND, 4, BF16, 576, 1, 1>(full, p, grid, threads, smem, st);
+        case 5: return launch_pipe_v<KIND, 5, BF16, 576, 1, 1>(full, p, grid, threads, smem, st);
+        case 6: return launch_pipe_v<KIND, 6, BF16, 576, 1, 1>(full, p, grid, threads, smem, st);
+        case 7: return launch_pipe_v<KIND, 7, BF16, 576, 1, 1>(full, p, grid, threads, smem, st);
+        case 8: return launch_pipe_v<KIND, 8, BF16, 576, 1, 1>(full, p, grid, threads, smem, st);
         default: return PB_UNSUPPORTED_SHAPE;
     }
-    if (rc) return rc;
-    PB_CUDA(cudaGetLastError());
-    return PB_OK;
 }
 
 constexpr int kPipeMinRows = 256;      // below this one CTA per row is as good (too few rows to pipeline)

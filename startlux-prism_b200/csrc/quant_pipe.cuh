@@ -55,17 +55,21 @@ __device__ __forceinline__ __nv_bfloat162 absmax_bf16x8(const uint4& u, __nv_bfl
     return m;
 }
 
-// The block size is chosen at launch so that blockDim.x * VPT just covers the row's vectors (a fixed size left up to
-// a quarter of the threads without a vector); MAXT bounds it for the register allocation.
-template <int KIND, int VPT, bool BF16, bool FULL, int MAXT>
-__global__ void __launch_bounds__(MAXT, 1)
+// The block size is chosen at launch so that a group's threads * VPT just cover the row's vectors (a fixed size left up to
+// a quarter of the threads without a vector); MAXT and MINB (CTAs per SM) bound it for the register allocation.
+// A row's time is a chain - its copy, the maximum over the block, the rounding - of which one group of threads works on one link
+// at a time, so several rows have to be in work per SM: MINB CTAs where rows are short, or, where a row fills a third
+// of shared memory, G groups of threads in one CTA that take alternate rows of one ring.
+template <int KIND, int VPT, bool BF16, bool FULL, int MAXT, int MINB, int G>
+__global__ void __launch_bounds__(MAXT, MINB)
 row_pipe_kernel(const PipeArgs p) {
-    const int THREADS = blockDim.x;
+    const int THREADS = blockDim.x / G, group = threadIdx.x / THREADS, tid = threadIdx.x - group * THREADS;
     extern __shared__ uint8_t pipe_smem_raw[];
     const uint32_t smem = (smem_u32(pipe_smem_raw) + 127u) & ~127u;
     __shared__ uint64_t full[8];
-    __shared__ float red[32];
+    __shared__ float red_all[G][32];
     __shared__ int abort_flag;
+    float* red = red_all[group];
     const int live = min(*p.n_rows, p.T);
     const int nvec = p.K >> 3;
     const int my_rows = live > (int)blockIdx.x ? (live - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
@@ -79,7 +83,7 @@ row_pipe_kernel(const PipeArgs p) {
         mbar_fence_init();
     }
     __syncthreads();
-    auto issue = [&](int i) {                    // thread 0: bulk copy of this CTA's i-th row into slot i % stages
+    auto issue = [&](int i) {                    // one thread: bulk copy of this CTA's i-th row into slot i % stages
         const long t = (long)blockIdx.x + (long)i * gridDim.x;
         const int s = i % p.stages;
         const uint32_t bar = smem_u32(&full[s]);
@@ -90,16 +94,20 @@ row_pipe_kernel(const PipeArgs p) {
                      : "memory");
     };
     if (threadIdx.x == 0)
-        for (int i = 0; i < p.stages - 1 && i < my_rows; ++i) issue(i);
+        for (int i = 0; i < p.stages && i < my_rows; ++i) issue(i);
+    auto group_sync = [&] {
+        if (G == 1) __syncthreads();
+        else if (group == 0) asm volatile("bar.sync 1, %0;" ::"r"(THREADS) : "memory");
+        else asm volatile("bar.sync 2, %0;" ::"r"(THREADS) : "memory");
+    };
 
     const bool smooth = p.inv_s != nullptr;
-    for (int i = 0; i < my_rows; ++i) {
+    bool ok = true;                              // a copy that never came: the rest of the loop stores nothing
+    for (int i = group; i < my_rows; i += G) {
         const long t = (long)blockIdx.x + (long)i * gridDim.x;
         const int s = i % p.stages;
-        // the slot of row i + stages - 1 was read by every thread in iteration i - 1 (the block barriers below)
-        if (threadIdx.x == 0 && i + p.stages - 1 < my_rows) issue(i + p.stages - 1);
-        if (!mbar_wait(smem_u32(&full[s]), (uint32_t)((i / p.stages) & 1), &abort_flag, 0xF00 + s)) break;
-        const uint32_t row = smem + (uint32_t)(s * p.row_bytes) + threadIdx.x * (BF16 ? 16u : 32u);
+        if (!mbar_wait(smem_u32(&full[s]), (uint32_t)((i / p.stages) & 1), &abort_flag, 0xF00 + s)) ok = false;
+        const uint32_t row = smem + (uint32_t)(s * p.row_bytes) + tid * (BF16 ? 16u : 32u);
         float v[VPT][8];
         uint4 raw[PACKED ? VPT : 1];
         float amax = 0.0f;
@@ -107,7 +115,7 @@ row_pipe_kernel(const PipeArgs p) {
             __nv_bfloat162 m2 = __float2bfloat162_rn(0.0f);
 #pragma unroll
             for (int j = 0; j < VPT; ++j) {
-                if (threadIdx.x + j * THREADS < nvec) {
+                if (tid + j * THREADS < nvec) {
                     raw[j] = lds128(row + j * THREADS * 16);
                     m2 = absmax_bf16x8(raw[j], m2);
                 }
@@ -116,7 +124,7 @@ row_pipe_kernel(const PipeArgs p) {
         } else {
 #pragma unroll
             for (int j = 0; j < VPT; ++j) {
-                const int c = threadIdx.x + j * THREADS;
+                const int c = tid + j * THREADS;
                 if (c < nvec) {
                     if (KIND == PIPE_SWIGLU) {
                         float g[8], u[8];
@@ -145,20 +153,25 @@ row_pipe_kernel(const PipeArgs p) {
                 }
             }
         }
-        amax = block_max(amax, red);             // two block barriers: every thread is done with slot s after them
-        if (p.mode == MODE_STORE_AMAX && threadIdx.x == 0) p.amax_io[t] = amax;
+        amax = warp_max(amax);
+        if ((tid & 31) == 0) red[tid >> 5] = amax;
+        group_sync();
+        if (tid == 0 && ok && i + p.stages < my_rows) issue(i + p.stages);   // every thread of the group is done with slot s
+        amax = warp_max((tid & 31) < (THREADS >> 5) ? red[tid & 31] : 0.0f);
+        group_sync();
+        if (p.mode == MODE_STORE_AMAX && tid == 0 && ok) p.amax_io[t] = amax;
         if (p.mode == MODE_USE_AMAX) amax = fmaxf(p.amax_io[t], amax);
         const float scale = fdiv<FULL>(fmaxf(amax, 1e-10f), 127.0f);
         const float rcp = __fdiv_rn(1.0f, scale);
-        int8_t* qrow = p.q + t * p.K + threadIdx.x * 8;
+        int8_t* qrow = p.q + t * p.K + tid * 8;
 #pragma unroll
         for (int j = 0; j < VPT; ++j) {
-            if (threadIdx.x + j * THREADS < nvec) {
+            if (tid + j * THREADS < nvec && ok) {
                 if (PACKED && !smooth) unpack_bf16x8(raw[j], v[j]);
                 *(uint2*)(qrow + j * THREADS * 8) = quant8<FULL>(v[j], scale, rcp);
             }
         }
-        if (threadIdx.x == 0) p.s[t] = scale;
+        if (tid == 0 && ok) p.s[t] = scale;
     }
     // armed copies of rows this CTA never reached (abort only) must land before the shared memory is released
     if (abort_flag && threadIdx.x == 0) {
