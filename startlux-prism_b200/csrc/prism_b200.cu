@@ -21,6 +21,7 @@
 #include "w4a8_gemv.cuh"
 #include "w4a8_mma.cuh"
 #include "w8a8_gemv.cuh"
+#include "w8a8_tpair.cuh"
 #include "mxfp4_gemm.cuh"
 #include "mxfp4_few.cuh"
 #include "mxfp4_gemv.cuh"
@@ -350,6 +351,53 @@ bool w4a8_tile_only() {
         v = (e && e[0] == '1') ? 1 : 0;
     }
     return v == 1;
+}
+
+// PRISM_B200_TPAIR=0: the single-CTA tile kernel for every many-row product (comparison runs).
+bool tpair_enabled() {
+    static int v = -1;
+    if (v < 0) {
+        const char* e = getenv("PRISM_B200_TPAIR");
+        v = (e && e[0] == '0') ? 0 : 1;
+    }
+    return v == 1;
+}
+
+// Activation rows of a row tile of w8a8_tpair_kernel: the fewest cycles by rounds of pairs, 256 + nt a stage (shared memory) and a
+// tile's drain that the last round does not hide.
+int tpair_rows(int M, int N, int K) {
+    const long KB = (K + 127) / 128, nn = (N + 255) / 256, pairs = sm_count() / 2;
+    int best = 0;
+    long cycles = 0;
+    for (int t = (M + 255) / 256, i = 0; i < 4; ++t, ++i) {
+        const int nt = ((M + t - 1) / t + 15) & ~15;
+        const long c = (nn * ((M + nt - 1) / nt) + pairs - 1) / pairs * (KB * (256 + nt) + 1500);
+        if (!best || c < cycles) {
+            best = nt;
+            cycles = c;
+        }
+    }
+    return best;
+}
+
+template <int EPI>
+int launch_tpair(const int8_t* a, const float* a_s, const int8_t* w, const float* w_s, void* out, long ldo, const int* n_rows, int M,
+                 int N, int K, cudaStream_t st) {
+    const int nt = tpair_rows(M, N, K);
+    CUtensorMap ta, tw;
+    int rc;
+    if ((rc = tensor_map(&ta, a, K, M, K, w8a8::BK, nt / 2, 0))) return rc;
+    if ((rc = tensor_map(&tw, w, K, N, K, w8a8::BK, w8a8::BM, 0))) return rc;
+    auto kern = w8a8::w8a8_tpair_kernel<EPI>;
+    static_assert(w8a8::TP_SMEM <= 232448, "shared memory of a CTA");
+    if ((rc = set_smem(kern, w8a8::TP_SMEM))) return rc;
+    const int tiles = ((M + nt - 1) / nt) * ((N + 255) / 256), pairs = sm_count() / 2;
+    // weight tiles fastest when the activations are the larger operand, do not fit in L2 and the weights do
+    const int n_fastest = (long)M * K > (long)N * K && (long)M * K > (64l << 20) && (long)N * K <= (100l << 20);
+    kern<<<2 * (tiles < pairs ? tiles : pairs), w8a8::TP_THREADS, w8a8::TP_SMEM, st>>>(tw, ta, a_s, w_s, out, ldo, n_rows, M, N, K, nt,
+                                                                                       n_fastest);
+    PB_CUDA(cudaGetLastError());
+    return PB_OK;
 }
 
 template <int EPI>
@@ -1044,6 +1092,14 @@ int pb_w8a8_gemm(const int8_t* a, const float* a_s, const int8_t* w, const float
             if (!workspace || !counters) return PB_BAD_ARGUMENT;
             if (workspace_bytes < pb_w8a8_workspace_bytes(M, N, split) || n_counters < pb_w8a8_counters(M, N))
                 return PB_TOO_LARGE;
+        }
+        // CTA pairs with the weights on the lanes.  One launch, us, against the tile kernel below (7168 x 5120 | 5120 x 5120 with residual add |
+        // 34816 x 5120 | 5120 x 17408 with residual add): 65 rows 14.2/15.9 | 14.8/14.0 | 35.2/38.6 | 33.5/47.4; 200 rows 16.2/16.4 |
+        // 15.3/15.6 | 40.6/48.2 | 35.8/36.4; 333 rows 18.5/22.6 | 16.4/15.7 | 54.9/61.6 | 37.9/36.9; 1,000 rows 29.8/39.9 | 26.2/36.1 |
+        // 118.8/138.0 | 71.9/106.9; 8,192 rows 186/208 | 147/170 | 877/959 | 488/553.
+        if (tpair_enabled() && epi != PB_EPI_I32 && !g_drop_loads) {
+            if (epi == PB_EPI_BF16) return launch_tpair<w8a8::EPI_BF16>(a, a_s, w, w_s, out, ldo, n_rows, M, N, K, st);
+            return launch_tpair<w8a8::EPI_ADD>(a, a_s, w, w_s, out, ldo, n_rows, M, N, K, st);
         }
         // tile width: 128 x 256, 128 x 128 when those would leave more than half of the SMs without a tile, or (one K
         // slice only) 128 x 192 when that needs fewer tile-widths of waves: 5120 columns at 2048 rows are 320 tiles
