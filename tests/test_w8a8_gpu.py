@@ -423,3 +423,24 @@ def test_dependent_reads_weight_scales_after_the_wait(dev, M, N, K):
             assert same(swd, sw) and same(out, bf16_from_bits(ref)), first_diff(np_bits(out), ref)
     finally:
         _lib.lib().pb_set_pdl(before)
+
+
+@pytest.mark.parametrize("M,N,K,live", [(65, 40, 144, 65), (81, 257, 128, 80), (177, 520, 912, 170), (257, 1000, 784, 257),
+                                        (1100, 300, 2192, 1031), (4200, 264, 1040, 4111), (16400, 256, 4112, 16399)])
+def test_many_rows_pair_tiles(dev, M, N, K, live):
+    """The CTA-pair kernel: row counts around its tiles of 16 to 256 rows, weight rows that end inside a CTA's 128, K that ends inside a
+    stage and goes around the ring, both tile orders; out a column slice at an odd offset.  The sums are exact in 64 bits, the
+    scales and the add one rounding each."""
+    a, w, sa, sw = (t.to(dev) for t in rand_w8a8(M, N, K, seed=M + N))
+    acc = (a.double() @ w.double().T).float()
+    ref = (acc * sa.view(-1, 1)) * sw.view(1, -1)
+    nr = n_rows(live, dev)
+    out = torch.full((M, N + 6), 3.0, dtype=torch.bfloat16, device=dev)
+    w8a8.gemm(a, sa.view(-1), w, sw.view(-1), out[:, 3:3 + N], nr, K)
+    assert same(out[:live, 3:3 + N].contiguous(), ref[:live].bfloat16())
+    base = torch.randn(M, N + 6, generator=torch.Generator().manual_seed(2)).to(dev)
+    res = base.clone()
+    w8a8.gemm(a, sa.view(-1), w, sw.view(-1), res[:, 1:1 + N], nr, K, epi=1)
+    assert same(res[:live, 1:1 + N].contiguous(), (base[:live, 1:1 + N] + ref[:live]).contiguous())
+    assert bool((out[live:] == 3).all()) and bool((out[:, :3] == 3).all()) and bool((out[:, 3 + N:] == 3).all())
+    assert same(res[live:], base[live:]) and same(res[:, :1], base[:, :1]) and same(res[:, 1 + N:], base[:, 1 + N:])
