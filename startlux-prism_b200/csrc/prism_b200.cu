@@ -673,6 +673,49 @@ int launch_w4a8(const int8_t* xq, const float* a, const int8_t* xs, int Ma, cons
     return PB_OK;
 }
 
+// More rows: operands expanded into tensor memory (w4a8_ts.cuh, tiles of 128 weight rows x 128 activation rows) or into shared memory
+// (w4a8_gemm.cuh, 64 x 128)?  By rounds of tiles over the SMs times a super-block's measured time, us: 1.2 (Q6_K 1.5) with up to
+// 64 activation rows and 1.65 (1.7) above against 1.07 (1.0).  50 rows of 34816 x 5120 48.5 against 87, of 5120 x 5120 26 against 23; 200 rows
+// of 5120 x 5120 35 against 43; 512 rows of 6144 x 5120 67 against 66; 2,048 rows of 34816 x 5120 944 against 1,240; Q6_K
+// 5120 x 17408 128 rows 116 against 70, 200 rows 118 against 136, 512 rows 229 against 204, 2,048 rows 563 against 610.
+bool w4a8_in_tmem(bool q4, int M, int N) {
+    const long sms = sm_count(), ts = (long)((M + 127) / 128) * ((N + 127) / 128), old = (long)((M + 127) / 128) * ((N + 63) / 64);
+    const long c_ts = M <= 64 ? (q4 ? 120 : 150) : q4 ? 165 : 170, c_old = q4 ? 107 : 100;
+    return (ts + sms - 1) / sms * c_ts < (old + sms - 1) / sms * c_old;
+}
+
+template <int KIND>
+int launch_w4a8_ts(const int8_t* xq, const float* a, const int8_t* xs, int Ma, const void* wq, const void* wsc,
+                   const void* wmn, const float* wd, const float* wdm, void* out, long ldo, const int* n_rows, int M,
+                   int N, int K, int epi, cudaStream_t st) {
+    using C = w4a8::TsCfg<KIND>;
+    constexpr int NBU = C::NBU, HMAX = C::HMAX;
+    static_assert(C::SMEM <= 232448, "shared memory of a CTA");
+    w4a8::TsMaps m;
+    int rc;
+    const uint64_t NSB = K / 256;
+    const int xbox = M < NBU ? (M + 15) & ~15 : NBU;
+    if ((rc = tensor_map(&m.x, xq, K, M, K, 128, xbox, 0))) return rc;
+    if (C::Q4) {
+        if ((rc = tensor_map(&m.wq, wq, K / 2, N, K / 2, 128, 128, 0))) return rc;
+        if ((rc = tensor_map(&m.xs, xs, (uint64_t)Ma * 4, NSB, (uint64_t)Ma * 16, NBU * 4, 1, 3))) return rc;
+        if ((rc = tensor_map(&m.sc, wsc, (uint64_t)N * 2, NSB, (uint64_t)N * 8, 256, 1, 3))) return rc;
+        if ((rc = tensor_map(&m.mn, wmn, (uint64_t)N * 2, NSB, (uint64_t)N * 8, 256, 1, 3))) return rc;
+    } else {
+        if ((rc = tensor_map(&m.wq, wq, K, N, K, 128, 128, 0))) return rc;
+        if ((rc = tensor_map(&m.sc, wsc, (uint64_t)N * 4, NSB, (uint64_t)N * 16, 256, 1, 3))) return rc;
+        m.xs = m.x;
+        m.mn = m.x;
+    }
+    auto kern = w4a8::w4a8_ts_kernel<KIND>;
+    if ((rc = set_smem(kern, C::SMEM))) return rc;
+    const w4a8::TsArgs p{a, wd, wdm, out, ldo, n_rows, M, N, K, Ma, epi, xbox};
+    const long tiles = (long)((M + NBU * HMAX - 1) / (NBU * HMAX)) * ((N + 127) / 128);
+    kern<<<(unsigned)(tiles < sm_count() ? tiles : sm_count()), C::THREADS, C::SMEM, st>>>(m, p);
+    PB_CUDA(cudaGetLastError());
+    return PB_OK;
+}
+
 // A decode batch (w4a8_mma.cuh).  Per configuration: 8 * MT activation rows, 16 * NT * WN weight rows and WK super-blocks a
 // round per CTA, ST rounds in flight.
 template <int KIND, int MT, int NT, int WN, int WK, int ST>
@@ -1609,6 +1652,10 @@ int pb_w4a8_gemm(const int8_t* xq, const float* a, const int8_t* xs, int Ma, int
         if (kind == 0) return launch_w4a8_few<w4a8::KIND_Q4K>(g, st);
         if (M == 2 && N > 16 * sm_count() && !w4a8_no_gemv()) return launch_w4a8_gemv<2>(kind, g, st);
         return launch_w4a8_few<w4a8::KIND_Q6K>(g, st);
+    }
+    if (w4a8_in_tmem(kind == 0, M, N)) {
+        if (kind == 0) return launch_w4a8_ts<w4a8::KIND_Q4K>(xq, a, xs, Ma, wq, wsc, wmn, wd, wdm, out, ldo, n_rows, M, N, K, epi, st);
+        return launch_w4a8_ts<w4a8::KIND_Q6K>(xq, a, xs, Ma, wq, wsc, wmn, wd, wdm, out, ldo, n_rows, M, N, K, epi, st);
     }
     if (kind == 0)
         return launch_w4a8<w4a8::KIND_Q4K>(xq, a, xs, Ma, wq, wsc, wmn, wd, wdm, out, ldo, n_rows, M, N, K, epi, st);

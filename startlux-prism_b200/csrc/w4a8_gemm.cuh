@@ -19,12 +19,11 @@
 // super-block the MMAs fill one of two accumulator sets in tensor memory while the epilogue warps drain the other
 // (the floating-point step per 256 inputs).
 #pragma once
-#include "common.cuh"
+#include "w4a8_ts.cuh"
 
 namespace w4a8 {
 
 constexpr int BM = 128, BN = 64;
-constexpr int KIND_Q4K = 0, KIND_Q6K = 1;
 
 template <int KIND>
 struct Cfg {
@@ -80,19 +79,6 @@ struct Args {
     const int* n_rows;
     int M, N, K, Ma, epi;
 };
-
-// K-major operand without swizzle: 8-row x 16-byte core matrices, `sbo` bytes between 8-row groups, `lbo` bytes
-// between the two 16-byte K chunks of a K = 32 step.
-__device__ __forceinline__ uint64_t umma_desc_plain(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr & 0x3FFFF) >> 4);
-    d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
-    d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
-    d |= (uint64_t)1 << 46;
-    return d;
-}
-
-__device__ __forceinline__ uint32_t swz(int row, int chunk) { return (uint32_t)(row * 128 + ((chunk ^ (row & 7)) << 4)); }
 
 // Q4_K: 32 packed inputs (16 bytes: low nibbles = inputs 0..15, high nibbles = inputs 16..31) times the 6-bit
 // sub-block scale, split s0 + 8 s1, into chunks 2j and 2j + 1 of rows n (plane 0) and 64 + n (plane 1).  A byte

@@ -117,6 +117,31 @@ def test_gemm_bits_long_k(dev, kind, m, live, n, k):
     assert bool((out[live:] == 3).all()) and bool((out[:, :3] == 3).all()) and bool((out[:, 3 + n:] == 3).all())
 
 
+@pytest.mark.parametrize("kind,m,live,n,k", [("q4k", 40, 33, 19000, 512), ("q4k", 200, 199, 5000, 768), ("q4k", 150, 129, 4996, 2304),
+                                             ("q4k", 300, 300, 13000, 512), ("q6k", 200, 193, 4900, 1280), ("q6k", 300, 290, 9900, 512),
+                                             ("q6k", 64, 49, 19004, 256)])
+def test_gemm_bits_tensor_memory_operand(dev, kind, m, live, n, k):
+    """Sizes that run with the expanded weights in tensor memory: one and two units of 64 rows a tile and part of one, a tile or more
+    per SM, weight rows that end inside a tile, K below and above its three stages."""
+    w, g = random_weights(kind, n, k, n + k + m)
+    at = torch.cat([torch.arange(140), torch.randint(0, n, (200,), generator=g), torch.arange(n - 140, n)])
+    pick = lambda t: None if t is None else t[:, at].contiguous()                        # noqa: E731
+    part = w4a8.W4(kind, w.q[at].contiguous(), pick(w.sc), pick(w.mn), pick(w.d), pick(w.dm), len(at), k)
+    xq, a, xs = oracle.quant_g(np_bits(synth.activations(m, k, seed=m, outliers=k // 64)))
+    base = torch.randn(m, n + 6, generator=g)
+    wd, nr = w.to(dev), n_rows(live, dev)
+    xqd, ad, xsd = (torch.from_numpy(t).to(dev) for t in (xq, a, xs))
+    out, res = torch.full((m, n + 6), 3.0, dtype=torch.bfloat16, device=dev), base.to(dev)
+    w4a8.gemm(xqd, ad, xsd, wd, out[:, 3:3 + n], nr)
+    w4a8.gemm(xqd, ad, xsd, wd, res[:, 1:1 + n], nr, epi=1)
+    out, res = out.cpu(), res.cpu()
+    ref0 = ref_gemm(xq, a, xs, part, 0, live)
+    ref1 = ref_gemm(xq, a, xs, part, 1, live, out=base[:, 1 + at].numpy())
+    assert np.array_equal(np_bits(out[:live, 3 + at]), ref0[:live]), first_diff(np_bits(out[:live, 3 + at]), ref0[:live])
+    assert same(res[:, 1 + at], ref1), first_diff(res[:, 1 + at].numpy(), ref1)
+    assert bool((out[live:] == 3).all()) and bool((out[:, :3] == 3).all()) and bool((out[:, 3 + n:] == 3).all())
+
+
 @pytest.mark.parametrize("kind,n,k", [("q4k", 1000, 1024), ("q4k", 8200, 768), ("q6k", 1000, 1024), ("q6k", 5000, 768)])
 def test_batch_invariance_across_kernels(dev, kind, n, k):
     """A row's bits do not depend on how many rows are multiplied with it, although 1, 2, 8, 9, 17, 33 and 100 rows run on
