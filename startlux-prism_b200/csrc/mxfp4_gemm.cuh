@@ -589,21 +589,23 @@ mxfp4_gemm256_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         if (elect_one()) {
             // MMA issuer.  The scale factors' copies into tensor memory are another thread's (warp 2): one thread doing
             // both issued twelve asynchronous instructions per K block, about 700 cycles against 570 of MMA time.
+            // The scale factors' barrier implies the stage's own (warp 2 waited for that before it copied them), and the next
+            // block's is asked for before this block's MMAs: a barrier test takes about 200 cycles to answer.
             int stage = 0;
-            uint32_t phase = 0, tphase = 0;
+            uint32_t tphase = 0;
             long kbt = 0;                                             // K blocks issued so far, over all tiles
-            bool ok = true;
+            bool ok = true, ready = false;
             for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
                 // one accumulator: the previous tile must be drained
                 if (!mbar_wait(smem_u32(&aux->tempty[0]), tphase ^ 1, abort_flag, 0x1710)) break;
                 tc_fence_after();
                 for (int kb = 0; kb < KB; ++kb, ++kbt) {
                     const int sfp = (int)(kbt & 1);
-                    if (!mbar_wait(smem_u32(&aux->full[stage]), phase, abort_flag, 0x1720 + stage) ||
-                        !mbar_wait(smem_u32(&aux->full[4 + sfp]), (uint32_t)(kbt >> 1) & 1, abort_flag, 0x1740 + sfp)) {
+                    if (!ready && !mbar_wait(smem_u32(&aux->full[4 + sfp]), (uint32_t)(kbt >> 1) & 1, abort_flag, 0x1740 + sfp)) {
                         ok = false;
                         break;
                     }
+                    ready = mbar_peek(smem_u32(&aux->full[4 + (sfp ^ 1)]), (uint32_t)((kbt + 1) >> 1) & 1);
                     tc_fence_after();
                     const uint32_t st = smem_u32(smem + stage * STAGE2_BYTES);
                     const uint32_t sfa_t = tmem_base + 256 + sfp * 24, sfb_t = sfa_t + 8;
@@ -616,10 +618,7 @@ mxfp4_gemm256_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                                   (kb | k) ? 1u : 0u);
                     }
                     tc_commit(smem_u32(&aux->empty[stage]));
-                    if (++stage == STAGES2) {
-                        stage = 0;
-                        phase ^= 1;
-                    }
+                    if (++stage == STAGES2) stage = 0;
                 }
                 if (!ok) break;
                 tc_commit(smem_u32(&aux->tfull[0]));
@@ -682,46 +681,66 @@ mxfp4_gemm256_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
                 // 32 rows x 64 bytes per chunk, parked densely in shared memory and handed to the copy engine: a plain
                 // tile store (bf16) or an add into the fp32 residual (one round-to-nearest add per element; the tensor
                 // map ends at row M and column N, so nothing outside is touched).  No load, no store loop.
-                if (m0 + q * 32 < p.M) {
-#pragma unroll 1
-                    for (int c0 = half * (BN2 / 2); c0 < (half + 1) * (BN2 / 2); c0 += cstep) {
-                        if (n0 + c0 >= p.N) break;
-                        uint32_t wv[16];
-                        if (p.epi == 0) {
-                            uint32_t r[32];
-                            tmem_ld32(lane_addr + c0, r);
-                            tmem_ld_wait();
+                // The accumulator is read into registers whole and handed back before anything is stored: the next tile's MMAs
+                // wait for it (there is one), and the boxes go out one after another through one buffer per warp (4,000 rows: 7168 x 5120
+                // 84 -> 70 us, 34816 x 5120 334 -> 298, 5120 x 17408 164 -> 166).
+                auto send = [&](int c0, const uint32_t* wv) {
+                    if (n0 + c0 >= p.N) return;
+                    // the engine must be done reading the box (the previous chunk) before it is rewritten
+                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    __syncwarp();
+                    uint4* dst = (uint4*)(stg + lane * 16);
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                __nv_bfloat162 b0 =
-                                    __floats2bfloat162_rn(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
-                                wv[j] = *(uint32_t*)&b0;
-                            }
-                        } else {
-                            tmem_ld16(lane_addr + c0, wv);
-                            tmem_ld_wait();
-                        }
-                        // the engine must be done reading the box (the previous chunk) before it is rewritten
-                        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                        __syncwarp();
-                        uint4* dst = (uint4*)(stg + lane * 16);
+                    for (int v = 0; v < 4; ++v) dst[v] = make_uint4(wv[4 * v], wv[4 * v + 1], wv[4 * v + 2], wv[4 * v + 3]);
+                    fence_async_smem();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (p.epi == 0)
+                            // (the bf16 output is described as 32-bit words: two columns per element)
+                            asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
+                                         : : "l"(&tm_out), "r"((n0 + c0) >> 1), "r"(m0 + q * 32), "r"(smem_u32(stg)) : "memory");
+                        else
+                            asm volatile(
+                                "cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];"
+                                : : "l"(&tm_out), "r"(n0 + c0), "r"(m0 + q * 32), "r"(smem_u32(stg)) : "memory");
+                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    }
+                };
+                auto give_back = [&] {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&aux->tempty[0]));
+                    tphase ^= 1;
+                };
+                const int cb = half * (BN2 / 2);
+                if (m0 + q * 32 >= p.M) {
+                    give_back();
+                } else if (p.epi == 0) {
+                    uint32_t wv[4][16];
 #pragma unroll
-                        for (int v = 0; v < 4; ++v) dst[v] = make_uint4(wv[4 * v], wv[4 * v + 1], wv[4 * v + 2], wv[4 * v + 3]);
-                        fence_async_smem();
-                        __syncwarp();
-                        if (lane == 0) {
-                            if (p.epi == 0)
-                                // (the bf16 output is described as 32-bit words: two columns per element)
-                                asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
-                                             : : "l"(&tm_out), "r"((n0 + c0) >> 1), "r"(m0 + q * 32), "r"(smem_u32(stg)) : "memory");
-                            else
-                                asm volatile(
-                                    "cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];"
-                                    : : "l"(&tm_out), "r"(n0 + c0), "r"(m0 + q * 32), "r"(smem_u32(stg)) : "memory");
-                            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    for (int i = 0; i < 4; ++i) {
+                        uint32_t r[32];
+                        tmem_ld32(lane_addr + cb + 32 * i, r);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            __nv_bfloat162 b0 = __floats2bfloat162_rn(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+                            wv[i][j] = *(uint32_t*)&b0;
                         }
                     }
+                    give_back();
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) send(cb + 32 * i, wv[i]);
+                } else {
+                    uint32_t wv[8][16];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) tmem_ld16(lane_addr + cb + 16 * i, wv[i]);
+                    tmem_ld_wait();
+                    give_back();
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) send(cb + 16 * i, wv[i]);
                 }
+                continue;
             } else {
 #pragma unroll 1
                 for (int c0 = half * (BN2 / 2); c0 < (half + 1) * (BN2 / 2); c0 += cstep) {
