@@ -1140,7 +1140,13 @@ int pb_w8a8_gemm(const int8_t* a, const float* a_s, const int8_t* w, const float
         // 34816 x 5120 | 5120 x 17408 with residual add): 65 rows 14.2/15.9 | 14.8/14.0 | 35.2/38.6 | 33.5/47.4; 200 rows 16.2/16.4 |
         // 15.3/15.6 | 40.6/48.2 | 35.8/36.4; 333 rows 18.5/22.6 | 16.4/15.7 | 54.9/61.6 | 37.9/36.9; 1,000 rows 29.8/39.9 | 26.2/36.1 |
         // 118.8/138.0 | 71.9/106.9; 8,192 rows 186/208 | 147/170 | 877/959 | 488/553.
-        if (tpair_enabled() && epi != PB_EPI_I32 && !g_drop_loads) {
+        // The tile kernel stays where its 128 x 128 tiles are half a wave to one and K is short enough for a pair's longer set-up and drain
+        // to show: 5120 x 5120 333 rows 15.7 against 16.4; 1024 x 5120 1,500 rows 15.6 against 17.1; 5120 x 2560 333 rows 10.4 against 12.3;
+        // for K up to 2560 from a quarter of a wave to two: 512 x 2048 1,500 rows 10.0 against 11.6; 5120 x 2560 700 rows 14.6 against
+        // 17.1 - but 1024 x 5120 333 rows 15.0 against 14.1, 5120 x 8704 333 rows 23.9 against 22.2.
+        const long t128 = (long)((M + 127) / 128) * ((N + 127) / 128);
+        const bool tile = K <= 2560 ? t128 * 4 >= sm_count() && t128 <= 2 * sm_count() : K <= 5120 && t128 * 2 >= sm_count() && t128 <= sm_count();
+        if (tpair_enabled() && !tile && epi != PB_EPI_I32 && !(epi == PB_EPI_ADD && add_mode() != 1) && !g_drop_loads) {
             if (epi == PB_EPI_BF16) return launch_tpair<w8a8::EPI_BF16>(a, a_s, w, w_s, out, ldo, n_rows, M, N, K, st);
             return launch_tpair<w8a8::EPI_ADD>(a, a_s, w, w_s, out, ldo, n_rows, M, N, K, st);
         }
