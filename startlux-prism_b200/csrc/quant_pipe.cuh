@@ -59,7 +59,8 @@ __device__ __forceinline__ __nv_bfloat162 absmax_bf16x8(const uint4& u, __nv_bfl
 // a quarter of the threads without a vector); MAXT and MINB (CTAs per SM) bound it for the register allocation.
 // A row's time is a chain - its copy, the maximum over the block, the rounding - of which one group of threads works on one link
 // at a time, so several rows have to be in work per SM: MINB CTAs where rows are short, or, where a row fills a third
-// of shared memory, G groups of threads in one CTA that take alternate rows of one ring.
+// of shared memory, G groups of threads in one CTA that take alternate rows of one ring.  The stack's pass at 8,192 rows 10,340 -> 10,170 us,
+// at 333 rows 791 -> 746 together with the elected issuers.
 template <int KIND, int VPT, bool BF16, bool FULL, int MAXT, int MINB, int G>
 __global__ void __launch_bounds__(MAXT, MINB)
 row_pipe_kernel(const PipeArgs p) {
