@@ -26,6 +26,7 @@ _SIGS = {
     "pb_device_status": ([ctypes.POINTER(_i), ctypes.POINTER(ctypes.c_uint), _i], _i),
     "pb_set_wait_limit_ns": ([ctypes.c_ulonglong], _i),
     "pb_test_drop_loads": ([_i], _i),
+    "pb_test_row_ring": ([_i, _i, _i, _vp, _vp, _vp], _i),
     "pb_w8a8_workspace_bytes": ([_i, _i, _i], _l),
     "pb_w8a8_counters": ([_i, _i], _i),
     "pb_w8a8_gemm": ([_vp, _vp, _vp, _vp, _vp, _l, _vp, _i, _i, _i, _i, _i, _i, _l, _vp, _l, _vp, _i, _i, _vp], _i),

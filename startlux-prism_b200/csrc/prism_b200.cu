@@ -878,6 +878,7 @@ bool w4a8_no_gemv() {
 template <int KIND, int VPT, bool BF16, int MAXT, int MINB, int G>
 int launch_pipe_v(bool full, const quant::PipeArgs& p, int grid, int threads, int smem, cudaStream_t st) {
     int rc;
+    if (G * p.stages > quant::RING_BARRIERS) return PB_UNSUPPORTED_SHAPE;
     auto k = full ? quant::row_pipe_kernel<KIND, VPT, BF16, true, MAXT, MINB, G> : quant::row_pipe_kernel<KIND, VPT, BF16, false, MAXT, MINB, G>;
     if ((rc = set_smem(k, 220 * 1024))) return rc;
     k<<<grid, threads, smem, st>>>(p);
@@ -1032,6 +1033,15 @@ int pb_set_pdl(int on) {
     const int before = g_pdl;
     g_pdl = on ? 1 : 0;
     return before;
+}
+
+int pb_test_row_ring(int groups, int stages, int row, int* slot, int* barrier, int* parity) {
+    const quant::RowRing ring{groups, stages};
+    if (groups < 1 || stages < 2 || ring.barriers() > quant::RING_BARRIERS || row < 0 || !slot || !barrier || !parity) return PB_BAD_ARGUMENT;
+    *slot = ring.slot(row);
+    *barrier = ring.barrier(row);
+    *parity = (int)ring.parity(row);
+    return PB_OK;
 }
 
 int pb_test_drop_loads(int on) {

@@ -55,6 +55,20 @@ __device__ __forceinline__ __nv_bfloat162 absmax_bf16x8(const uint4& u, __nv_bfl
     return m;
 }
 
+// The ring of a CTA's rows.  Row i lies in slot i % stages; its copy is counted on a barrier of its own sequence, rows that are
+// groups * stages apart.  With groups of threads taking alternate rows, a barrier per slot would pass from group to group when the slots
+// are not a multiple of the groups: a wait knows the phase's parity only, so a group that asks for row i + stages while row i's
+// copy is still in flight (another group's row) is told yes at once.  Here all rows of a barrier are one group's, and a row
+// is armed after the row two turns before it was waited for: a wait is never more than one phase ahead of its barrier.
+struct RowRing {
+    int groups, stages;
+    __host__ __device__ int slot(int i) const { return i % stages; }
+    __host__ __device__ int barriers() const { return groups * stages; }
+    __host__ __device__ int barrier(int i) const { return i % (groups * stages); }
+    __host__ __device__ uint32_t parity(int i) const { return (uint32_t)(i / (groups * stages)) & 1u; }
+};
+constexpr int RING_BARRIERS = 8;
+
 // The block size is chosen at launch so that a group's threads * VPT just cover the row's vectors (a fixed size left up to
 // a quarter of the threads without a vector); MAXT and MINB (CTAs per SM) bound it for the register allocation.
 // A row's time is a chain - its copy, the maximum over the block, the rounding - of which one group of threads works on one link
@@ -67,7 +81,8 @@ row_pipe_kernel(const PipeArgs p) {
     const int THREADS = blockDim.x / G, group = threadIdx.x / THREADS, tid = threadIdx.x - group * THREADS;
     extern __shared__ uint8_t pipe_smem_raw[];
     const uint32_t smem = (smem_u32(pipe_smem_raw) + 127u) & ~127u;
-    __shared__ uint64_t full[8];
+    const RowRing ring{G, p.stages};
+    __shared__ uint64_t full[RING_BARRIERS];
     __shared__ float red_all[G][32];
     __shared__ int abort_flag;
     float* red = red_all[group];
@@ -79,15 +94,15 @@ row_pipe_kernel(const PipeArgs p) {
     constexpr bool PACKED = KIND == PIPE_ROWS && BF16;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < p.stages; ++s) mbar_init(smem_u32(&full[s]), 1);
+        for (int b = 0; b < ring.barriers(); ++b) mbar_init(smem_u32(&full[b]), 1);
         abort_flag = 0;
         mbar_fence_init();
     }
     __syncthreads();
-    auto issue = [&](int i) {                    // one thread: bulk copy of this CTA's i-th row into slot i % stages
+    auto issue = [&](int i) {                    // one thread: bulk copy of this CTA's i-th row into its slot
         const long t = (long)blockIdx.x + (long)i * gridDim.x;
-        const int s = i % p.stages;
-        const uint32_t bar = smem_u32(&full[s]);
+        const int s = ring.slot(i);
+        const uint32_t bar = smem_u32(&full[ring.barrier(i)]);
         mbar_expect_tx(bar, (uint32_t)p.row_bytes);
         const uint8_t* src = (const uint8_t*)p.x + t * p.ldx * (BF16 ? 2 : 4);
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -106,9 +121,8 @@ row_pipe_kernel(const PipeArgs p) {
     bool ok = true;                              // a copy that never came: the rest of the loop stores nothing
     for (int i = group; i < my_rows; i += G) {
         const long t = (long)blockIdx.x + (long)i * gridDim.x;
-        const int s = i % p.stages;
-        if (!mbar_wait(smem_u32(&full[s]), (uint32_t)((i / p.stages) & 1), &abort_flag, 0xF00 + s)) ok = false;
-        const uint32_t row = smem + (uint32_t)(s * p.row_bytes) + tid * (BF16 ? 16u : 32u);
+        if (!mbar_wait(smem_u32(&full[ring.barrier(i)]), ring.parity(i), &abort_flag, 0xF00 + ring.barrier(i))) ok = false;
+        const uint32_t row = smem + (uint32_t)(ring.slot(i) * p.row_bytes) + tid * (BF16 ? 16u : 32u);
         float v[VPT][8];
         uint4 raw[PACKED ? VPT : 1];
         float amax = 0.0f;
@@ -157,7 +171,7 @@ row_pipe_kernel(const PipeArgs p) {
         amax = warp_max(amax);
         if ((tid & 31) == 0) red[tid >> 5] = amax;
         group_sync();
-        if (tid == 0 && ok && i + p.stages < my_rows) issue(i + p.stages);   // every thread of the group is done with slot s
+        if (tid == 0 && ok && i + p.stages < my_rows) issue(i + p.stages);   // every thread of the group is done with the slot
         amax = warp_max((tid & 31) < (THREADS >> 5) ? red[tid & 31] : 0.0f);
         group_sync();
         if (p.mode == MODE_STORE_AMAX && tid == 0 && ok) p.amax_io[t] = amax;

@@ -171,6 +171,69 @@ def test_argument_checks_without_gpu(lib):
     assert lib.pb_mxfp4_gemv(p16, p16, p16, p16, p16, 128, 1, 128, 128, 0, None) == 2                # K % 256
 
 
+def _run_row_ring(where, groups, stages, rows, rng):
+    """The row quantizers' loop over a CTA's rows with copies that land in any order and groups that run at any speed: `where(row)` is
+    (slot, barrier, parity).  Returns what went wrong, or None.  A wait is true when the barrier's phase has the other parity."""
+    slots, phase, armed, flying = [None] * stages, {}, set(), []
+    at, waiting = list(range(groups)), [True] * groups
+
+    def issue(i):
+        slot, bar, _ = where(i)
+        if bar in armed:
+            return f"row {i} arms a barrier whose copy is still in flight"
+        armed.add(bar)
+        slots[slot] = ("copy in flight", i)
+        flying.append(i)
+
+    for i in range(min(stages, rows)):
+        issue(i)
+    for _ in range(100 * rows):
+        g = rng.randrange(groups + 1)
+        if g == groups:                                   # a copy lands
+            if flying:
+                i = flying.pop(rng.randrange(len(flying)))
+                slot, bar, _ = where(i)
+                slots[slot] = ("row", i)
+                armed.discard(bar)
+                phase[bar] = phase.get(bar, 0) + 1
+        elif at[g] < rows:
+            slot, bar, parity = where(at[g])
+            if waiting[g]:
+                if phase.get(bar, 0) & 1 != parity:
+                    waiting[g] = False                    # it reads from here on
+                    if slots[slot] != ("row", at[g]):
+                        return f"row {at[g]} read while its slot holds {slots[slot]}"
+            else:
+                wrong = issue(at[g] + stages) if at[g] + stages < rows else None
+                if wrong:
+                    return wrong
+                at[g] += groups
+                waiting[g] = True
+    return None if min(at) >= rows else f"stuck at {at}"
+
+
+@pytest.mark.parametrize("groups,stages", [(1, 2), (1, 3), (1, 8), (2, 2), (2, 3), (2, 4)])
+def test_row_ring_waits_for_its_own_copy(lib, groups, stages):
+    """Whatever order the copies land in, a row is read after its own copy, and no barrier is armed twice.  One barrier per
+    slot does not give that when the slots are not a multiple of the groups, which the model has to see."""
+    import random
+
+    def where(i):
+        out = [ctypes.c_int() for _ in range(3)]
+        assert lib.pb_test_row_ring(groups, stages, i, *(ctypes.addressof(x) for x in out)) == 0
+        return tuple(x.value for x in out)
+
+    per_slot = lambda i: (i % stages, i % stages, (i // stages) & 1)                         # noqa: E731
+    rows = [where(i) for i in range(64)]
+    assert all(0 <= s < stages and 0 <= b < 8 for s, b, _ in rows)
+    for seed in range(300):
+        assert _run_row_ring(rows.__getitem__, groups, stages, 40 + seed % 20, random.Random(seed)) is None
+    seen = any(_run_row_ring(per_slot, groups, stages, 60, random.Random(seed)) for seed in range(300))
+    assert seen == (stages % groups != 0)
+    n = ctypes.addressof(ctypes.c_int())
+    assert lib.pb_test_row_ring(2, 5, 0, n, n, n) == 1 and lib.pb_test_row_ring(1, 9, 0, n, n, n) == 1
+
+
 def test_split_rules_of_the_other_formats():
     from prism_b200 import mxfp4, w4a8
     # few-rows W4A8: time goes as waves / slices; Q6_K's 80 tiles of the down projection take 7 slices (4 waves)

@@ -212,6 +212,25 @@ def test_swiglu_q8_many_rows(dev, T, FF):
     assert same(q2, q[:200].contiguous()) and same(s2, s[:200].contiguous())
 
 
+@pytest.mark.parametrize("T,FF,live", [(2003, 17408, 1990), (2500, 13608, 2500), (2100, 13832, 2011), (1900, 17920, 1900)])
+def test_swiglu_q8_ring_turns(dev, T, FF, live):
+    """Twelve and more rows per CTA: the two groups of threads go around rings of three and four slots more than once, so every slot passes
+    between them.  Every mode's bytes and scales are those of the one-CTA-per-row kernel on slices below 256 rows."""
+    g = torch.Generator(device=dev).manual_seed(FF)
+    gu = (torch.randn(T, 2 * FF, generator=g, device=dev) * 2).bfloat16()
+    inv = torch.rand(FF, generator=g, device=dev) + 0.5
+    for mode, smooth in ((0, None), (0, inv), (1, None), (2, None)):
+        q, q2 = (torch.full((T, FF), 99, dtype=torch.int8, device=dev) for _ in range(2))
+        s, s2 = (torch.full((T,), -1.0, device=dev) for _ in range(2))
+        amax, amax2 = (torch.arange(T, device=dev).float() % 50 if mode == 2 else torch.zeros(T, device=dev) for _ in range(2))
+        kw = lambda a: dict(mode=mode, amax=a) if mode else {}                               # noqa: E731
+        quant.swiglu_q8(gu, smooth, q, s, n_rows(live, dev), T, **kw(amax))
+        for r in range(0, live, 250):
+            n = min(250, live - r)
+            quant.swiglu_q8(gu[r:r + n], smooth, q2[r:r + n], s2[r:r + n], n_rows(n, dev), n, **kw(amax2[r:r + n]))
+        assert same(q, q2) and same(s, s2) and same(amax, amax2), (mode, smooth is None)
+
+
 @pytest.mark.parametrize("T,HID,live", [(7, 5120, 5), (64, 5120, 64), (33, 2048, 33), (3, 17408, 3)])
 def test_norm_q8(dev, T, HID, live):
     """RMSNorm + per-token int8 (kernels/quant.py:145-171): within one int8 step of the oracle (the sum of squares has
