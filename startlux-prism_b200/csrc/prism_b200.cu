@@ -363,14 +363,15 @@ bool tpair_enabled() {
     return v == 1;
 }
 
-// Activation rows of a row tile of w8a8_tpair_kernel: the fewest cycles by rounds of pairs, 256 + nt a stage (shared memory) and a
-// tile's drain that the last round does not hide.
+// Activation rows of a row tile of w8a8_tpair_kernel, which are N of its MMA: a multiple of 32, the only sizes that int8 MMAs of a CTA
+// pair have (one CTA's go in steps of 16).  The fewest cycles by rounds of pairs, 256 + nt a stage (shared memory) and a tile's
+// drain that the last round does not hide.
 int tpair_rows(int M, int N, int K) {
     const long KB = (K + 127) / 128, nn = (N + 255) / 256, pairs = sm_count() / 2;
     int best = 0;
     long cycles = 0;
     for (int t = (M + 255) / 256, i = 0; i < 4; ++t, ++i) {
-        const int nt = ((M + t - 1) / t + 15) & ~15;
+        const int nt = ((M + t - 1) / t + 31) & ~31;
         const long c = (nn * ((M + nt - 1) / nt) + pairs - 1) / pairs * (KB * (256 + nt) + 1500);
         if (!best || c < cycles) {
             best = nt;
@@ -386,6 +387,7 @@ int launch_tpair(const int8_t* a, const float* a_s, const int8_t* w, const float
     const int nt = tpair_rows(M, N, K);
     CUtensorMap ta, tw;
     int rc;
+    if (nt % 32 || nt < 32 || nt > w8a8::TP_MAX) return PB_UNSUPPORTED_SHAPE;
     if ((rc = tensor_map(&ta, a, K, M, K, w8a8::BK, nt / 2, 0))) return rc;
     if ((rc = tensor_map(&tw, w, K, N, K, w8a8::BK, w8a8::BM, 0))) return rc;
     auto kern = w8a8::w8a8_tpair_kernel<EPI>;
@@ -1067,6 +1069,8 @@ long pb_w8a8_workspace_bytes(int M, int N, int split) {
     const long tiles = (long)((N + 127) / 128) * ((M + nb - 1) / nb);
     return (long)split * tiles * nb * 128 * 4;
 }
+
+int pb_w8a8_pair_rows(int M, int N, int K) { return M <= 0 || N <= 0 || K <= 0 ? 0 : tpair_rows(M, N, K); }
 
 int pb_w8a8_counters(int M, int N) {
     if (M <= 0 || N <= 0) return 0;

@@ -1,6 +1,6 @@
 // W8A8 GEMM for more than 64 rows (gk == K) on CTA pairs with the operands exchanged.  The weight rows are the MMA's M operand (256 of
-// them, 128 per CTA and tensor-memory lane set), the activation rows its N: a row tile is any multiple of 16 up to 256, so
-// 333 rows are two tiles of 176 where tiles of 128 rows compute 384.
+// them, 128 per CTA and tensor-memory lane set), the activation rows its N: a row tile is any multiple of 32 up to 256, the sizes
+// that an int8 MMA of a CTA pair has.
 // What bounds w8a8_tile_kernel is shared memory: an MMA of 128 x 256 x 32 on one CTA reads 12 KB in 128 cycles while the copy
 // engine writes as much for the coming ones, 192 bytes a clock where an SM moves 128.  A pair reads and is sent half of the
 // activation tile per CTA: (256 + nt) cycles a stage by that count, 512 at nt = 256 - the MMAs' own time there.

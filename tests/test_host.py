@@ -234,6 +234,14 @@ def test_row_ring_waits_for_its_own_copy(lib, groups, stages):
     assert lib.pb_test_row_ring(2, 5, 0, n, n, n) == 1 and lib.pb_test_row_ring(1, 9, 0, n, n, n) == 1
 
 
+def test_pair_tiles_are_shapes_of_the_mma(lib):
+    """Row tiles of the CTA-pair kernel are N of an int8 MMA of two CTAs, which exists in steps of 32 up to 256."""
+    for n, k in ((7168, 5120), (5120, 17408), (34816, 5120), (512, 2048), (40, 144), (100000, 4096)):
+        for m in [*range(65, 1200), 2047, 2048, 4097, 8191, 8192, 16400, 100000]:
+            nt = lib.pb_w8a8_pair_rows(m, n, k)
+            assert nt % 32 == 0 and 32 <= nt <= 256, (m, n, k, nt)
+
+
 def test_split_rules_of_the_other_formats():
     from prism_b200 import mxfp4, w4a8
     # few-rows W4A8: time goes as waves / slices; Q6_K's 80 tiles of the down projection take 7 slices (4 waves)
