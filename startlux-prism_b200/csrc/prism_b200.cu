@@ -1138,8 +1138,8 @@ int pb_w8a8_gemm(const int8_t* a, const float* a_s, const int8_t* w, const float
         return launch_pair<w8a8::EPI_ADD>(a, a_s, w, w_s, out, ldo, n_rows, M, N, K, st);
     }
     if (M > 64) {
-        // many rows: K splits (few tiles only: callers pick them, w8a8.pick_split) add their int32 partial sums in a
-        // workspace, exactly; the last CTA of a tile runs the epilogue
+        // many rows: K splits (few tiles only: callers pick them, w8a8.pick_split) run on the tile kernel and add their int32
+        // partial sums in a workspace, exactly; the last CTA of a tile runs the epilogue
         if (split > KB) split = KB;
         if (split > 1) {
             const int kbs = (KB + split - 1) / split;
@@ -1160,7 +1160,7 @@ int pb_w8a8_gemm(const int8_t* a, const float* a_s, const int8_t* w, const float
         // 17.1 - but 1024 x 5120 333 rows 15.0 against 14.1, 5120 x 8704 333 rows 23.9 against 22.2.
         const long t128 = (long)((M + 127) / 128) * ((N + 127) / 128);
         const bool tile = K <= 2560 ? t128 * 4 >= sm_count() && t128 <= 2 * sm_count() : K <= 5120 && t128 * 2 >= sm_count() && t128 <= sm_count();
-        if (tpair_enabled() && !tile && epi != PB_EPI_I32 && !(epi == PB_EPI_ADD && add_mode() != 1) && !g_drop_loads) {
+        if (tpair_enabled() && split == 1 && !tile && epi != PB_EPI_I32 && !(epi == PB_EPI_ADD && add_mode() != 1) && !g_drop_loads) {
             if (epi == PB_EPI_BF16) return launch_tpair<w8a8::EPI_BF16>(a, a_s, w, w_s, out, ldo, n_rows, M, N, K, st);
             return launch_tpair<w8a8::EPI_ADD>(a, a_s, w, w_s, out, ldo, n_rows, M, N, K, st);
         }

@@ -10,8 +10,8 @@
 gk == K (the engine's mode): one scale per token and per output channel; every kernel, K split and batch size gives an
 output element the same bits: v = (float(acc) * a_s[m]) * w_s[n], each product rounded, epi 1 adds with one more
 rounding.  gk == 32 uses Q8_0's own block scales: fp32 partial products added in group order.
-Kernel choice (this module's table replaces the reference's per-GPU JSON tables): more than 64 rows -> the persistent
-128 x 256 tile kernel; up to 64 rows -> the operand-swapped split-K kernel, the splits' int32 sums either deferred to
+Kernel choice (this module's table replaces the reference's per-GPU JSON tables): more than 64 rows -> the CTA-pair
+kernel or the persistent tile kernel (the library's rule; K splits on the latter); up to 64 rows -> the operand-swapped split-K kernel, the splits' int32 sums either deferred to
 the caller's `slots` (epi 1) or added inside the kernel through a workspace.
 """
 import math
@@ -106,8 +106,9 @@ GEMV_ROWS = 1        # gk == K: this many rows against few weight rows run on th
 def pick_split(M, N, K, limit=MAX_SPLIT):
     """K splits.  Few rows (operand-swapped kernel): as many CTAs as stay resident together, at least two 128-byte K
     blocks each.  Many rows (tile kernel, one CTA per SM): only when the 128 x 256 tiles leave most SMs idle and K is
-    long (at least 32 K blocks per slice; measured: a gain for K = 17408 at 128-256 rows, a loss for K = 5120) - the
-    slices' int32 sums meet in the workspace, exactly."""
+    long (at least 32 K blocks per slice) - the slices' int32 sums meet in the workspace, exactly.  gemm splits bf16 products only:
+    1024 x 17408 at 128 rows takes 21.1 us in four slices, 32.1 unsplit, but a residual add 37.1 and 32.3 - the last CTA of a
+    tile waits for what it adds to."""
     kb = -(-K // 128)
     if M > FEW_ROWS:
         tiles = -(-M // 128) * -(-N // 256)
@@ -221,7 +222,7 @@ def gemm(a, a_s, w, w_s, out, n_rows, gk, epi=0, outs=None, cfg=None, slots=None
     elif M <= FEW_ROWS:
         split, defer_ok = _few_split(M, N, K, epi == EPI_ADD, pdl and scratch is not None)
     else:
-        split = pick_split(M, N, K)
+        split = pick_split(M, N, K) if epi == EPI_BF16 else 1
     split = effective_split(K, split)
     if split > 1 and M <= FEW_ROWS and epi == EPI_ADD and slots is not None and slots.shape[1] >= M and defer_ok:
         split = effective_split(K, min(split, slots.shape[0]))

@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import oracle
-from prism_b200 import quant, w8a8
+from prism_b200 import _lib, quant, w8a8
 from util import bf16_from_bits, first_diff, n_rows, np_bits, rand_w8a8, same
 
 pytestmark = pytest.mark.gpu
@@ -444,3 +444,20 @@ def test_many_rows_pair_tiles(dev, M, N, K, live):
     assert same(res[:live, 1:1 + N].contiguous(), (base[:live, 1:1 + N] + ref[:live]).contiguous())
     assert bool((out[live:] == 3).all()) and bool((out[:, :3] == 3).all()) and bool((out[:, 3 + N:] == 3).all())
     assert same(res[live:], base[live:]) and same(res[:, :1], base[:, :1]) and same(res[:, 1 + N:], base[:, 1 + N:])
+
+
+@pytest.mark.parametrize("M,N,K,split", [(100, 512, 17408, 4), (333, 1000, 6144, 3), (700, 300, 1040, 2)])
+def test_many_rows_split_is_run(dev, M, N, K, split):
+    """A K split asked for above 64 rows is the one that runs: the slices meet in the caller's workspace, the counters are left zero and the
+    bits are the unsplit product's."""
+    a, w, sa, sw = (t.to(dev) for t in rand_w8a8(M, N, K, seed=M + split))
+    sa, sw, nr = sa.view(-1), sw.view(-1), n_rows(M, dev)
+    L = _lib.lib()
+    for epi, dtype in ((0, torch.bfloat16), (1, torch.float32)):
+        want, out = (torch.full((M, N), 0.5, dtype=dtype, device=dev) for _ in range(2))
+        w8a8._call(a, sa, w, sw, want, N, nr, K, epi, 1)
+        ws = torch.full((L.pb_w8a8_workspace_bytes(M, N, split),), 0x55, dtype=torch.uint8, device=dev)
+        counters = torch.zeros(L.pb_w8a8_counters(M, N), dtype=torch.int32, device=dev)
+        w8a8._call(a, sa, w, sw, out, N, nr, K, epi, split, 0, ws, counters)
+        assert same(out, want)
+        assert bool((ws != 0x55).any()) and not bool(counters.any())
