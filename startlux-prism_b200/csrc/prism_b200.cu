@@ -390,10 +390,16 @@ int launch_tpair(const int8_t* a, const float* a_s, const int8_t* w, const float
     if (nt % 32 || nt < 32 || nt > w8a8::TP_MAX) return PB_UNSUPPORTED_SHAPE;
     if ((rc = tensor_map(&ta, a, K, M, K, w8a8::BK, nt / 2, 0))) return rc;
     if ((rc = tensor_map(&tw, w, K, N, K, w8a8::BK, w8a8::BM, 0))) return rc;
-    auto kern = w8a8::w8a8_tpair_kernel<EPI>;
+    const int tiles = ((M + nt - 1) / nt) * ((N + 255) / 256), pairs = sm_count() / 2;
+    // Residual adds in registers where the copy engine could not address the output either, and where a K split, which adds in registers,
+    // is what few tiles of long K would otherwise be: there a tile has few rows (1024 x 17408, us: 31.2 -> 31.3 with 32 rows a tile,
+    // 5120 x 17408 at 128 rows 35.0 -> 35.8 with 64).  Elsewhere the reduction is faster: 5120 x 5120 333 rows 16.7 against 17.8, 4,096 rows
+    // 80.9 against 92.
+    const long t128 = (long)((M + 127) / 128) * ((N + 127) / 128);
+    const bool regs = EPI == w8a8::EPI_ADD && (!aligned16(out) || ldo % 4 || (2 * t128 <= sm_count() && K > 63 * 128));
+    auto kern = regs ? w8a8::w8a8_tpair_kernel<EPI, EPI == w8a8::EPI_ADD> : w8a8::w8a8_tpair_kernel<EPI, false>;
     static_assert(w8a8::TP_SMEM <= 232448, "shared memory of a CTA");
     if ((rc = set_smem(kern, w8a8::TP_SMEM))) return rc;
-    const int tiles = ((M + nt - 1) / nt) * ((N + 255) / 256), pairs = sm_count() / 2;
     // weight tiles fastest when the activations are the larger operand, do not fit in L2 and the weights do
     const int n_fastest = (long)M * K > (long)N * K && (long)M * K > (64l << 20) && (long)N * K <= (100l << 20);
     kern<<<2 * (tiles < pairs ? tiles : pairs), w8a8::TP_THREADS, w8a8::TP_SMEM, st>>>(tw, ta, a_s, w_s, out, ldo, n_rows, M, N, K, nt,

@@ -16,7 +16,9 @@ constexpr int TP_STAGE_BYTES = BM * BK + TP_MAX / 2 * BK;         // per CTA: 12
 constexpr int TP_SMEM = TP_STAGES * TP_STAGE_BYTES + 1024 + (int)sizeof(Aux) + 2 * TP_MAX * 4;
 constexpr int TP_THREADS = 64 + 8 * 32;
 
-template <int EPI>
+// REGS (residual add): read, one rounded add, write, 16 rows requested ahead - before the products are there, for the first ones.
+// Otherwise a reduction at the memory side, for which nothing waits, but which flushes values below 2^-126.
+template <int EPI, bool REGS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
 w8a8_tpair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_a, const float* __restrict__ a_s,
                   const float* __restrict__ w_s, void* __restrict__ out, long ldo, const int* __restrict__ n_rows, int M, int N,
@@ -135,8 +137,7 @@ w8a8_tpair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         }
     } else {
         // ------------------------------------------------------------------ epilogue: 8 warps, two per lane quarter, half of the
-        // columns each; a lane holds one output column, so a warp's store of a row is 32 neighbouring columns.  The residual
-        // add is a reduction at the memory side (one rounded add per element, nothing waits for it), as in the tile kernel.
+        // columns each; a lane holds one output column, so a warp's store of a row is 32 neighbouring columns
         const int q = warp & 3, half = (warp - 2) >> 2, et = threadIdx.x - 64;
         int buf = 0;
         uint32_t bphase = 0;
@@ -145,14 +146,19 @@ w8a8_tpair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
             float* sab = sa_stash + buf * TP_MAX;
             for (int i = et; i < nt; i += 256) sab[i] = m0 + i < live ? a_s[m0 + i] : 0.0f;
             const float sw = n < N ? w_s[n] : 0.0f;
+            const int c1 = (half + 1) * (nt / 2);                        // nt / 2: a multiple of 16
+            float h0[16], h1[16];
+            auto fetch = [&](int c0, float (&h)[16]) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    if (c0 < c1 && m0 + c0 + j < live && n < N) h[j] = __ldcg((const float*)out + (long)(m0 + c0 + j) * ldo + n);
+            };
+            if (REGS) fetch(half * (nt / 2), h0);
             asm volatile("bar.sync 1, 256;" ::: "memory");
             if (!mbar_wait(smem_u32(&aux->tfull[buf]), bphase, abort_flag, 0x1C00 + buf)) break;
             tc_fence_after();
             const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + buf * TP_MAX;
-            const int c1 = (half + 1) * (nt / 2);
-#pragma unroll 1
-            for (int c0 = half * (nt / 2); c0 < c1; c0 += 8) {
-                if (m0 + c0 >= live) break;
+            auto rows8 = [&](int c0, const float* h) {
                 uint32_t r[8];
                 tmem_ld8(lane_addr + c0, r);
                 const float4 s0 = *(const float4*)(sab + c0), s1 = *(const float4*)(sab + c0 + 4);
@@ -164,10 +170,27 @@ w8a8_tpair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
                         if (m0 + c0 + j >= live) continue;
                         const float v = scale2((int)r[j], sa[j], sw);
                         const long at = (long)(m0 + c0 + j) * ldo + n;
-                        if (EPI == EPI_ADD) atomicAdd((float*)out + at, v);
+                        if (EPI == EPI_ADD && REGS) ((float*)out)[at] = __fadd_rn(h[j], v);
+                        else if (EPI == EPI_ADD) atomicAdd((float*)out + at, v);
                         else ((__nv_bfloat16*)out)[at] = __float2bfloat16_rn(v);
                     }
                 }
+            };
+            if (REGS) {
+#pragma unroll 1
+                for (int c0 = half * (nt / 2); c0 < c1 && m0 + c0 < live; c0 += 32) {
+                    fetch(c0 + 16, h1);
+                    rows8(c0, h0);
+                    rows8(c0 + 8, h0 + 8);
+                    fetch(c0 + 32, h0);
+                    if (c0 + 16 < c1) {
+                        rows8(c0 + 16, h1);
+                        rows8(c0 + 24, h1 + 8);
+                    }
+                }
+            } else {
+#pragma unroll 1
+                for (int c0 = half * (nt / 2); c0 < c1 && m0 + c0 < live; c0 += 8) rows8(c0, nullptr);
             }
             tc_fence_before();
             __syncwarp();

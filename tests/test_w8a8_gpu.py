@@ -461,3 +461,23 @@ def test_many_rows_split_is_run(dev, M, N, K, split):
         w8a8._call(a, sa, w, sw, out, N, nr, K, epi, split, 0, ws, counters)
         assert same(out, want)
         assert bool((ws != 0x55).any()) and not bool(counters.any())
+
+
+@pytest.mark.parametrize("M,N,K,off", [(100, 512, 17408, 0), (200, 640, 1040, 1), (1100, 5121, 272, 3), (333, 5120, 5120, 2)])
+def test_many_rows_add_keeps_subnormals(dev, M, N, K, off):
+    """Residual adds into an output that the copy engine cannot address (odd offset or stride), or of one round of tiles that share a long K,
+    are plain rounded adds: values below 2^-126 and sums there are kept."""
+    a, w, sa, sw = rand_w8a8(M, N, K, seed=M + off)
+    sa, sw = sa.view(-1) * 2.0 ** -60, sw.view(-1) * 2.0 ** -70
+    g = torch.Generator().manual_seed(off)
+    base = (torch.randint(-2 ** 20, 2 ** 20, (M, N + 2 * off), generator=g).double() * 2.0 ** -147).float()
+    res, nr = base.to(dev), n_rows(M, dev)
+    w8a8.gemm(a.to(dev), sa.to(dev), w.to(dev), sw.to(dev), res[:, off:off + N], nr, K, epi=1)
+    acc = (a.to(dev).double() @ w.to(dev).double().T).cpu().float()
+    v = (acc.double() * sa.double().view(-1, 1)).float()
+    v = (v.double() * sw.double()).float()                # rounded as fp32 products are, below 2^-126 too
+    ref = base.clone()
+    ref[:, off:off + N] = (base[:, off:off + N].double() + v.double()).float()
+    tiny = (ref.abs() < 2.0 ** -126) & (ref != 0)
+    assert int(tiny.sum()) > M * N // 2
+    assert same(res, ref), first_diff(res.cpu().numpy(), ref.numpy())
