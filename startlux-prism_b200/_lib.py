@@ -28,7 +28,7 @@ _SIGS = {
     "pb_test_drop_loads": ([_i], _i),
     "pb_test_row_ring": ([_i, _i, _i, _vp, _vp, _vp], _i),
     "pb_w8a8_workspace_bytes": ([_i, _i, _i], _l),
-    "pb_w8a8_pair_rows": ([_i, _i, _i], _i),
+    "pb_w8a8_pair_rows": ([_i, _i, _i, _i], _i),
     "pb_w8a8_counters": ([_i, _i], _i),
     "pb_w8a8_gemm": ([_vp, _vp, _vp, _vp, _vp, _l, _vp, _i, _i, _i, _i, _i, _i, _l, _vp, _l, _vp, _i, _i, _vp], _i),
     "pb_w8a8_gemm_swiglu": ([_vp, _vp, _vp, _vp, _vp, _l, _vp, _vp, _i, _i, _i, _i, _vp], _i),

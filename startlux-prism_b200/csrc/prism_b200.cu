@@ -363,22 +363,85 @@ bool tpair_enabled() {
     return v == 1;
 }
 
-// Activation rows of a row tile of w8a8_tpair_kernel, which are N of its MMA: a multiple of 32, the only sizes that int8 MMAs of a CTA
-// pair have (one CTA's go in steps of 16).  The fewest cycles by rounds of pairs, 256 + nt a stage (shared memory) and a tile's
-// drain that the last round does not hide.
+// Cycles of w8a8_tpair_kernel with row tiles of nt: rounds of pairs, each as long as its stages or the drain of the tile before, and the
+// last drain.  Fitted to 26 projections at 65 to 4,096 rows: a stage's MMAs take 2.06 nt, its copies and barriers 355 + nt / 4; with
+// more rounds the copies of all pairs bound it at 256 + nt; a row of a tile drains in 42.
+long tpair_cycles(int M, int N, int K, int nt) {
+    const long KB = (K + 127) / 128, pairs = sm_count() / 2;
+    const long rounds = ((long)((N + 255) / 256) * ((M + nt - 1) / nt) + pairs - 1) / pairs;
+    long stage = 206l * nt / 100;
+    if (stage < 355 + nt / 4) stage = 355 + nt / 4;
+    if (rounds > 1 && stage < 256 + nt) stage = 256 + nt;
+    const long drain = 42 * nt, main = KB * stage;
+    return (rounds - 1) * (main > drain ? main : drain) + main + drain;
+}
+
+// Activation rows of a row tile, which are N of its MMA: a multiple of 32, the only sizes that int8 MMAs of a CTA pair have (one CTA's
+// go in steps of 16).
 int tpair_rows(int M, int N, int K) {
-    const long KB = (K + 127) / 128, nn = (N + 255) / 256, pairs = sm_count() / 2;
     int best = 0;
     long cycles = 0;
-    for (int t = (M + 255) / 256, i = 0; i < 4; ++t, ++i) {
-        const int nt = ((M + t - 1) / t + 31) & ~31;
-        const long c = (nn * ((M + nt - 1) / nt) + pairs - 1) / pairs * (KB * (256 + nt) + 1500);
+    for (int nt = w8a8::TP_MAX; nt >= 32; nt -= 32) {
+        if (nt >= M + 32) continue;
+        const long c = tpair_cycles(M, N, K, nt);
         if (!best || c < cycles) {
             best = nt;
             cycles = c;
         }
     }
     return best;
+}
+
+// Weight rows per tile of w8a8_tile_kernel with K splits.
+int tile_bn(int M, int N) {
+    if (N <= 128) return 128;
+    const long tiles256 = (long)((M + 127) / 128) * ((N + 255) / 256);
+    return tiles256 * 2 <= sm_count() ? 128 : 256;
+}
+
+// In one K slice: 256, 128 when 256-wide tiles would leave more than half of the SMs without a tile, or 192 when that needs fewer
+// tile-widths of waves: 5120 columns at 2048 rows are 320 tiles of 256 = 3 waves x 256, but 432 tiles of 192 = 3 waves x 192.
+int tile_width(int M, int N, int split) {
+    if (N <= 128 || tile_bn(M, N) == 128) return 128;
+    if (split == 1 && wide192_enabled()) {
+        const long mt = (M + 127) / 128, sms = sm_count();
+        const long w256 = (mt * ((N + 255) / 256) + sms - 1) / sms * 256 * 100;
+        const long w192 = (mt * ((N + 191) / 192) + sms - 1) / sms * 192 * 107;     // its operand traffic per MMA is higher
+        if (w192 < w256) return 192;
+    }
+    return 256;
+}
+
+// Cycles of w8a8_tile_kernel as tpair_cycles counts them: waves of stages, and what its set-up and last drain take beyond the pair
+// kernel's - little for a residual add, which the copy engine makes.
+long tile_cycles(int M, int N, int K, bool add) {
+    const int bn = tile_width(M, N, 1);
+    const long sms = sm_count(), waves = ((long)((M + 127) / 128) * ((N + bn - 1) / bn) + sms - 1) / sms;
+    return waves * ((K + 127) / 128) * (bn == 128 ? 396 : bn == 192 ? 620 : 760) + (add ? 1000 : bn == 128 ? 4200 : 7000);
+}
+
+// Residual adds in registers where the copy engine could not address the output either, and where a K split, which adds in registers,
+// is what few tiles of long K would otherwise be: there a tile has few rows (1024 x 17408, us: 31.2 -> 31.3 with 32 rows a tile,
+// 5120 x 17408 at 128 rows 35.0 -> 35.8 with 64).  Elsewhere the reduction is faster: 5120 x 5120 333 rows 16.7 against 17.8, 4,096 rows
+// 80.9 against 92.
+bool add_addressable(const void* out, long ldo) { return aligned16(out) && ldo % 4 == 0; }
+bool tpair_add_regs(const void* out, long ldo, int M, int N, int K) {
+    const long t128 = (long)((M + 127) / 128) * ((N + 127) / 128);
+    return !add_addressable(out, ldo) || (2 * t128 <= sm_count() && K > 63 * 128);
+}
+
+// CTA pairs, or the tile kernel?  The shorter by the two counts above.  The 26 projections against the better of the two kernels
+// at its best row tile: 0.1 % behind on average, one more than 5 % (512 x 17408 4,096 rows 38.1 us against 35.9); ten others at 80 to
+// 8,192 rows 0.4 %.  The tile kernel is the
+// better one mostly for residual adds in one wave: 5120 x 5120 333 rows 14.7 against 16.7, 700 rows 21.6 against 23.3, 5120 x 17408 333 rows
+// 36.4 against 38.6, 5120 x 2560 500 rows 12.9 against 14.5.  Adds in registers stay on pairs (5120 x 5120 1,000 rows at an odd offset 30.7
+// against 40.2), but for short K in many rounds (10240 x 2560 2,048 rows 90.6 against 79.3).
+bool tpair_faster(const void* out, long ldo, int M, int N, int K, int epi) {
+    if (epi == PB_EPI_ADD && tpair_add_regs(out, ldo, M, N, K)) {
+        const int nt = tpair_rows(M, N, K);
+        return K > 2560 || (long)((N + 255) / 256) * ((M + nt - 1) / nt) <= 3 * (sm_count() / 2);
+    }
+    return tpair_cycles(M, N, K, tpair_rows(M, N, K)) <= tile_cycles(M, N, K, epi == PB_EPI_ADD);
 }
 
 template <int EPI>
@@ -391,12 +454,7 @@ int launch_tpair(const int8_t* a, const float* a_s, const int8_t* w, const float
     if ((rc = tensor_map(&ta, a, K, M, K, w8a8::BK, nt / 2, 0))) return rc;
     if ((rc = tensor_map(&tw, w, K, N, K, w8a8::BK, w8a8::BM, 0))) return rc;
     const int tiles = ((M + nt - 1) / nt) * ((N + 255) / 256), pairs = sm_count() / 2;
-    // Residual adds in registers where the copy engine could not address the output either, and where a K split, which adds in registers,
-    // is what few tiles of long K would otherwise be: there a tile has few rows (1024 x 17408, us: 31.2 -> 31.3 with 32 rows a tile,
-    // 5120 x 17408 at 128 rows 35.0 -> 35.8 with 64).  Elsewhere the reduction is faster: 5120 x 5120 333 rows 16.7 against 17.8, 4,096 rows
-    // 80.9 against 92.
-    const long t128 = (long)((M + 127) / 128) * ((N + 127) / 128);
-    const bool regs = EPI == w8a8::EPI_ADD && (!aligned16(out) || ldo % 4 || (2 * t128 <= sm_count() && K > 63 * 128));
+    const bool regs = EPI == w8a8::EPI_ADD && tpair_add_regs(out, ldo, M, N, K);
     auto kern = regs ? w8a8::w8a8_tpair_kernel<EPI, EPI == w8a8::EPI_ADD> : w8a8::w8a8_tpair_kernel<EPI, false>;
     static_assert(w8a8::TP_SMEM <= 232448, "shared memory of a CTA");
     if ((rc = set_smem(kern, w8a8::TP_SMEM))) return rc;
@@ -1057,13 +1115,6 @@ int pb_test_drop_loads(int on) {
     return PB_OK;
 }
 
-// Weight rows per tile of the many-rows kernel.
-int tile_bn(int M, int N) {
-    if (N <= 128) return 128;
-    const long tiles256 = (long)((M + 127) / 128) * ((N + 255) / 256);
-    return tiles256 * 2 <= sm_count() ? 128 : 256;
-}
-
 long pb_w8a8_workspace_bytes(int M, int N, int split) {
     if (M <= 0 || N <= 0 || split <= 1) return 0;
     if (M > 64) {                                       // tile kernel: int32 [tiles][split][128][BN]
@@ -1076,7 +1127,10 @@ long pb_w8a8_workspace_bytes(int M, int N, int split) {
     return (long)split * tiles * nb * 128 * 4;
 }
 
-int pb_w8a8_pair_rows(int M, int N, int K) { return M <= 0 || N <= 0 || K <= 0 ? 0 : tpair_rows(M, N, K); }
+int pb_w8a8_pair_rows(int M, int N, int K, int epi) {
+    if (M <= 64 || N <= 0 || K <= 0 || (epi != PB_EPI_BF16 && epi != PB_EPI_ADD)) return 0;
+    return tpair_faster(nullptr, 0, M, N, K, epi) ? tpair_rows(M, N, K) : 0;
+}
 
 int pb_w8a8_counters(int M, int N) {
     if (M <= 0 || N <= 0) return 0;
@@ -1156,30 +1210,12 @@ int pb_w8a8_gemm(const int8_t* a, const float* a_s, const int8_t* w, const float
             if (workspace_bytes < pb_w8a8_workspace_bytes(M, N, split) || n_counters < pb_w8a8_counters(M, N))
                 return PB_TOO_LARGE;
         }
-        // CTA pairs with the weights on the lanes.  One launch, us, against the tile kernel below (7168 x 5120 | 5120 x 5120 with residual add |
-        // 34816 x 5120 | 5120 x 17408 with residual add): 65 rows 14.2/15.9 | 14.8/14.0 | 35.2/38.6 | 33.5/47.4; 200 rows 16.2/16.4 |
-        // 15.3/15.6 | 40.6/48.2 | 35.8/36.4; 333 rows 18.5/22.6 | 16.4/15.7 | 54.9/61.6 | 37.9/36.9; 1,000 rows 29.8/39.9 | 26.2/36.1 |
-        // 118.8/138.0 | 71.9/106.9; 8,192 rows 186/208 | 147/170 | 877/959 | 488/553.
-        // The tile kernel stays where its 128 x 128 tiles are half a wave to one and K is short enough for a pair's longer set-up and drain
-        // to show: 5120 x 5120 333 rows 15.7 against 16.4; 1024 x 5120 1,500 rows 15.6 against 17.1; 5120 x 2560 333 rows 10.4 against 12.3;
-        // for K up to 2560 from a quarter of a wave to two: 512 x 2048 1,500 rows 10.0 against 11.6; 5120 x 2560 700 rows 14.6 against
-        // 17.1 - but 1024 x 5120 333 rows 15.0 against 14.1, 5120 x 8704 333 rows 23.9 against 22.2.
-        const long t128 = (long)((M + 127) / 128) * ((N + 127) / 128);
-        const bool tile = K <= 2560 ? t128 * 4 >= sm_count() && t128 <= 2 * sm_count() : K <= 5120 && t128 * 2 >= sm_count() && t128 <= sm_count();
-        if (tpair_enabled() && split == 1 && !tile && epi != PB_EPI_I32 && !(epi == PB_EPI_ADD && add_mode() != 1) && !g_drop_loads) {
+        if (tpair_enabled() && split == 1 && epi != PB_EPI_I32 && !(epi == PB_EPI_ADD && add_mode() != 1) && !g_drop_loads &&
+            tpair_faster(out, ldo, M, N, K, epi)) {
             if (epi == PB_EPI_BF16) return launch_tpair<w8a8::EPI_BF16>(a, a_s, w, w_s, out, ldo, n_rows, M, N, K, st);
             return launch_tpair<w8a8::EPI_ADD>(a, a_s, w, w_s, out, ldo, n_rows, M, N, K, st);
         }
-        // tile width: 128 x 256, 128 x 128 when those would leave more than half of the SMs without a tile, or (one K
-        // slice only) 128 x 192 when that needs fewer tile-widths of waves: 5120 columns at 2048 rows are 320 tiles
-        // of 256 = 3 waves x 256, but 432 tiles of 192 = 3 waves x 192
-        int bn = (N <= 128 || tile_bn(M, N) == 128) ? 128 : 256;
-        if (bn == 256 && split == 1 && wide192_enabled()) {
-            const long mt = (M + 127) / 128, sms = sm_count();
-            const long w256 = (mt * ((N + 255) / 256) + sms - 1) / sms * 256 * 100;
-            const long w192 = (mt * ((N + 191) / 192) + sms - 1) / sms * 192 * 107;     // its operand traffic per MMA is higher
-            if (w192 < w256) bn = 192;
-        }
+        const int bn = tile_width(M, N, split);
 #define PB_TILE(BN_, EPI_) launch_tile<BN_, w8a8::EPI_>(a, a_s, w, w_s, out, ldo, n_rows, M, N, K, st, split, workspace, counters, nullptr, nullptr, 0, workspace_bytes, n_counters)
         if (epi == PB_EPI_I32) return bn == 128 ? PB_TILE(128, EPI_I32) : bn == 192 ? PB_TILE(192, EPI_I32) : PB_TILE(256, EPI_I32);
         if (epi == PB_EPI_BF16) return bn == 128 ? PB_TILE(128, EPI_BF16) : bn == 192 ? PB_TILE(192, EPI_BF16) : PB_TILE(256, EPI_BF16);

@@ -235,11 +235,19 @@ def test_row_ring_waits_for_its_own_copy(lib, groups, stages):
 
 
 def test_pair_tiles_are_shapes_of_the_mma(lib):
-    """Row tiles of the CTA-pair kernel are N of an int8 MMA of two CTAs, which exists in steps of 32 up to 256."""
+    """Row tiles of the CTA-pair kernel are N of an int8 MMA of two CTAs, which exists in steps of 32 up to 256 (0: the tile kernel
+    runs)."""
     for n, k in ((7168, 5120), (5120, 17408), (34816, 5120), (512, 2048), (40, 144), (100000, 4096)):
         for m in [*range(65, 1200), 2047, 2048, 4097, 8191, 8192, 16400, 100000]:
-            nt = lib.pb_w8a8_pair_rows(m, n, k)
-            assert nt % 32 == 0 and 32 <= nt <= 256, (m, n, k, nt)
+            for epi in (0, 1):
+                nt = lib.pb_w8a8_pair_rows(m, n, k, epi)
+                assert nt % 32 == 0 and 0 <= nt <= 256, (m, n, k, nt)
+    assert lib.pb_w8a8_pair_rows(333, 34816, 5120, 0) == 192 and lib.pb_w8a8_pair_rows(8192, 34816, 5120, 0) == 256
+    # few weight rows: tiles small enough that the pairs fill the GPU (22 of 74 with 192 rows a tile)
+    assert lib.pb_w8a8_pair_rows(2048, 512, 5120, 0) == 64
+    # one wave of the tile kernel, whose copy engine makes the residual add
+    assert lib.pb_w8a8_pair_rows(333, 5120, 17408, 1) == 0 and lib.pb_w8a8_pair_rows(333, 5120, 5120, 1) == 0
+    assert lib.pb_w8a8_pair_rows(64, 5120, 5120, 0) == 0 and lib.pb_w8a8_pair_rows(333, 5120, 5120, 3) == 0
 
 
 def test_split_rules_of_the_other_formats():

@@ -426,11 +426,13 @@ def test_dependent_reads_weight_scales_after_the_wait(dev, M, N, K):
 
 
 @pytest.mark.parametrize("M,N,K,live", [(65, 40, 144, 65), (81, 257, 128, 80), (177, 520, 912, 170), (257, 1000, 784, 257),
-                                        (1100, 300, 2192, 1031), (4200, 100, 1040, 4111), (16400, 256, 4112, 16399)])
+                                        (1100, 300, 2192, 1031), (4200, 100, 1040, 4111), (16400, 256, 4112, 16399),
+                                        (300, 10240, 528, 299), (1000, 5000, 1296, 993), (1000, 9000, 3088, 993)])
 def test_many_rows_pair_tiles(dev, M, N, K, live):
-    """The CTA-pair kernel: row counts around its tiles of 16 to 256 rows, weight rows that end inside a CTA's 128, K that ends inside a
-    stage and goes around the ring, both tile orders; out a column slice at an odd offset.  The sums are exact in 64 bits, the
-    scales and the add one rounding each."""
+    """The CTA-pair kernel: row counts around its tiles of 32 to 256 rows, weight rows that end inside a CTA's 128, K that ends inside a
+    stage and goes around the ring, one round of tiles and more, both tile orders; out a column slice at an odd offset (adds in
+    registers) and whole (reductions).  The sums are exact in 64 bits, the scales and the add one rounding each."""
+    assert _lib.lib().pb_w8a8_pair_rows(M, N, K, 0)
     a, w, sa, sw = (t.to(dev) for t in rand_w8a8(M, N, K, seed=M + N))
     acc = (a.double() @ w.double().T).float()
     ref = (acc * sa.view(-1, 1)) * sw.view(1, -1)
@@ -444,6 +446,11 @@ def test_many_rows_pair_tiles(dev, M, N, K, live):
     assert same(res[:live, 1:1 + N].contiguous(), (base[:live, 1:1 + N] + ref[:live]).contiguous())
     assert bool((out[live:] == 3).all()) and bool((out[:, :3] == 3).all()) and bool((out[:, 3 + N:] == 3).all())
     assert same(res[live:], base[live:]) and same(res[:, :1], base[:, :1]) and same(res[:, 1 + N:], base[:, 1 + N:])
+    if N % 4 == 0 and _lib.lib().pb_w8a8_pair_rows(M, N, K, 1):
+        base = base[:, :N].contiguous()
+        res = base.clone()
+        w8a8.gemm(a, sa.view(-1), w, sw.view(-1), res, nr, K, epi=1)
+        assert same(res[:live], base[:live] + ref[:live]) and same(res[live:], base[live:])
 
 
 @pytest.mark.parametrize("M,N,K,split", [(100, 512, 17408, 4), (333, 1000, 6144, 3), (700, 300, 1040, 2)])
