@@ -224,7 +224,8 @@ int set_smem(Kernel k, int bytes) {
     return set_smem_raw((const void*)k, bytes);
 }
 
-// Failure injection from the host (pb_test_drop_loads): the many-rows W8A8 kernel's producers request no tiles.
+// Failure injection from the host (pb_test_drop_loads): the producers of the many-rows W8A8 tile kernel (1, which then runs every
+// product above 64 rows) or of the CTA-pair kernel (2) request no tiles.
 int g_drop_loads = 0;
 
 // ------------------------------------------------------------------------------------------------- W8A8 launches
@@ -307,7 +308,7 @@ int launch_tile(const int8_t* a, const float* a_s, const int8_t* w, const float*
     } else if (EPI == w8a8::EPI_ADD && whole_tiles && add_mode() == 2) {
         word_ok |= 4;
     }
-    if (g_drop_loads) word_ok |= 16;                               // failure injection (pb_test_drop_loads)
+    if (g_drop_loads == 1) word_ok |= 16;                               // failure injection (pb_test_drop_loads)
     // weight tiles fastest when the activations are the larger operand, do not fit in L2 and the weights do
     if ((long)M * K > (long)N * K && (long)M * K > (64l << 20) && (long)N * K <= (100l << 20)) word_ok |= 8;
     const int kbs = (KB + split - 1) / split;
@@ -461,7 +462,7 @@ int launch_tpair(const int8_t* a, const float* a_s, const int8_t* w, const float
     // weight tiles fastest when the activations are the larger operand, do not fit in L2 and the weights do
     const int n_fastest = (long)M * K > (long)N * K && (long)M * K > (64l << 20) && (long)N * K <= (100l << 20);
     kern<<<2 * (tiles < pairs ? tiles : pairs), w8a8::TP_THREADS, w8a8::TP_SMEM, st>>>(tw, ta, a_s, w_s, out, ldo, n_rows, M, N, K, nt,
-                                                                                       n_fastest);
+                                                                                       n_fastest | (g_drop_loads == 2 ? 2 : 0));
     PB_CUDA(cudaGetLastError());
     return PB_OK;
 }
@@ -1111,7 +1112,7 @@ int pb_test_row_ring(int groups, int stages, int row, int* slot, int* barrier, i
 }
 
 int pb_test_drop_loads(int on) {
-    g_drop_loads = on ? 1 : 0;
+    g_drop_loads = on == 2 ? 2 : on ? 1 : 0;
     return PB_OK;
 }
 
@@ -1210,7 +1211,7 @@ int pb_w8a8_gemm(const int8_t* a, const float* a_s, const int8_t* w, const float
             if (workspace_bytes < pb_w8a8_workspace_bytes(M, N, split) || n_counters < pb_w8a8_counters(M, N))
                 return PB_TOO_LARGE;
         }
-        if (tpair_enabled() && split == 1 && epi != PB_EPI_I32 && !(epi == PB_EPI_ADD && add_mode() != 1) && !g_drop_loads &&
+        if (tpair_enabled() && split == 1 && epi != PB_EPI_I32 && !(epi == PB_EPI_ADD && add_mode() != 1) && g_drop_loads != 1 &&
             tpair_faster(out, ldo, M, N, K, epi)) {
             if (epi == PB_EPI_BF16) return launch_tpair<w8a8::EPI_BF16>(a, a_s, w, w_s, out, ldo, n_rows, M, N, K, st);
             return launch_tpair<w8a8::EPI_ADD>(a, a_s, w, w_s, out, ldo, n_rows, M, N, K, st);

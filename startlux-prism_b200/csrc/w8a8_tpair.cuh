@@ -22,7 +22,8 @@ template <int EPI, bool REGS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
 w8a8_tpair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_a, const float* __restrict__ a_s,
                   const float* __restrict__ w_s, void* __restrict__ out, long ldo, const int* __restrict__ n_rows, int M, int N,
-                  int K, int nt, int n_fastest) {
+                  int K, int nt, int flags) {
+    const int n_fastest = flags & 1;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = align1024(smem_raw);
     Aux* aux = (Aux*)(smem + TP_STAGES * TP_STAGE_BYTES);
@@ -70,7 +71,7 @@ w8a8_tpair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
             const uint32_t tx = (uint32_t)(2 * (BM + nt / 2) * BK);              // both CTAs' bytes
             int stage = 0;
             uint32_t phase = 0;
-            bool ok = true;
+            bool ok = !(flags & 2);                              // failure injection from the host: nothing is requested
             for (int t = pair; t < num_tiles && ok; t += npairs) {
                 const int m0 = tile_m(t) + (int)rank * (nt / 2), n0 = tile_n(t) + (int)rank * BM;
                 for (int kb = 0; kb < KB; ++kb) {

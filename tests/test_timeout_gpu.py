@@ -45,3 +45,29 @@ def test_wait_expires_status_4_then_clean_launch(dev, lib):
     w8a8.gemm(ad, sad, wd, swd, out3, nr, K, cfg=2)
     torch.cuda.synchronize()
     assert same(out2, want) and same(out3, want)
+
+
+@pytest.mark.parametrize("epi", [0, 1])
+def test_pair_kernel_wait_expires(dev, lib, epi):
+    """The same on the CTA-pair kernel: both CTAs of a pair leave, whichever of them holds the barrier that nothing completes."""
+    M, N, K = 1000, 9000, 3088
+    assert lib.pb_w8a8_pair_rows(M, N, K, epi) == 256
+    a, w, sa, sw = (t.to(dev) for t in rand_w8a8(M, N, K, seed=12))
+    nr, dtype = n_rows(M, dev), (torch.bfloat16, torch.float32)[epi]
+    want, junk, out = (torch.full((M, N), 0.5, dtype=dtype, device=dev) for _ in range(3))
+    w8a8.gemm(a, sa.view(-1), w, sw.view(-1), want, nr, K, epi=epi)
+    assert _lib.device_status(reset=True)[0] == 0
+    assert lib.pb_set_wait_limit_ns(2_000_000) == 0
+    assert lib.pb_test_drop_loads(2) == 0
+    try:
+        w8a8.gemm(a, sa.view(-1), w, sw.view(-1), junk, nr, K, epi=epi)
+        torch.cuda.synchronize()                                     # returns: the waits were bounded
+        code, where = _lib.device_status(reset=True)
+    finally:
+        lib.pb_test_drop_loads(0)
+        lib.pb_set_wait_limit_ns(0)
+    assert code == 4 and where & 0xFF00 in (0x1B00, 0x1C00), (code, hex(where))
+    assert bool((junk == 0.5).all())                                 # nothing was stored from sums that never were
+    w8a8.gemm(a, sa.view(-1), w, sw.view(-1), out, nr, K, epi=epi)   # tensor memory was given back, the barriers are new
+    torch.cuda.synchronize()
+    assert same(out, want) and _lib.device_status(reset=False)[0] == 0
