@@ -299,13 +299,13 @@ def run_gpu(args):
             achieved = ops / world / (gemm_ms * 1e-3) / 1e12    # per GPU: this rank's share of the products / its GEMM time
             peak, peak_mean = int8_peak
             # DRAM bytes per launch of the dominant kernel (the gate|up GEMM): its algorithmic bytes (weights once +
-            # activations + bf16 output) times the ratio ncu measured on the one-launch capture at M = 2048 (300 MB of
-            # DRAM traffic against 332 MB algorithmic: part of the output was still in L2 when the capture ended)
+            # activations + bf16 output) times the ratio ncu measured on the one-launch capture at M = 2048 (305 MB of
+            # DRAM traffic against 331 MB algorithmic: part of the output was still in L2 when the capture ended)
             n_gu, k_gu = 34816 // world, 5120
             algorithmic = n_gu * k_gu + M * k_gu + 2 * M * n_gu
             line["roofline"] = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                                "frac": achieved / peak, "traffic": int(algorithmic * 0.90),
-                                "kernel": "w8a8_tile_kernel<256>", "gemm_ms_per_step": gemm_ms,
+                                "frac": achieved / peak, "traffic": int(algorithmic * 0.92),
+                                "kernel": "w8a8_tpair_kernel", "gemm_ms_per_step": gemm_ms,
                                 "algorithmic_bytes": algorithmic,
                                 "peak_note": "int8 tensor-core rate measured in this process before the timed region: "
                                              "tcgen05 kind::i8 128x256x32 on shared-memory-resident random operands, "
@@ -314,7 +314,7 @@ def run_gpu(args):
                                              f"{2 * pk['bf16_burst']:.0f}, 2 x sustained = {2 * pk['bf16']:.0f}, nominal "
                                              "dense int8 4500",
                                 "frac_of_nominal_4500": achieved / 4500.0,
-                                "traffic_note": "algorithmic bytes x 0.90, the DRAM / algorithmic ratio of the ncu "
+                                "traffic_note": "algorithmic bytes x 0.92, the DRAM / algorithmic ratio of the ncu "
                                                 "capture at M = 2048; not measured at this M"}
             if achieved > peak:
                 line["roofline"]["flag"] = "achieved above the measured peak: the probe ran at a lower clock than the step"
@@ -807,7 +807,7 @@ def run_probe(args):
         return run_peak(dev)
     ri = lambda *s: torch.randint(-127, 128, s, dtype=torch.int8, device=dev, generator=gen)     # noqa: E731
     if case in ("tile", "tile_add", "decode", "decode32", "config0"):
-        M = 2048 if case.startswith("tile") else 16
+        M = args.probe_rows or (2048 if case.startswith("tile") else 16)
         N, K = (34816, 5120) if case in ("tile", "decode32") else (5120, 17408)
         if case == "tile_add":
             N, K = 5120, 17408
@@ -824,7 +824,7 @@ def run_probe(args):
         fn = lambda: w8a8.gemm(a, sa, w, sw, out, nr, gk, epi=epi, slots=slots)                   # noqa: E731
         ops, nbytes = 2.0 * M * N * K, N * K + M * K
     elif case in ("w4a8_q4k", "w4a8_q6k", "w4a8_q4k_decode", "w4a8_q6k_decode"):
-        M, N, K = (args.probe_rows or 16, 34816, 5120) if case.endswith("decode") else (2048, 8192, 5120)
+        M, N, K = (args.probe_rows or 16, 34816, 5120) if case.endswith("decode") else (args.probe_rows or 2048, 8192, 5120)
         wcpu = synth.weights(N, K, 3)
         w = w4a8.repack((synth.q4_k if "q4k" in case else synth.q6_k)(wcpu)).to(dev)
         x = torch.randn(M, K, device=dev, generator=gen).to(torch.bfloat16)
@@ -837,7 +837,7 @@ def run_probe(args):
         fn = lambda: w4a8.gemm(q, s, xs, w, out, nr)                                              # noqa: E731
         ops, nbytes = 2.0 * M * N * K, w.nbytes() + M * K
     elif case == "mxfp4":
-        M, N, K = 2048, 34816, 5120
+        M, N, K = args.probe_rows or 2048, 34816, 5120
         wq = torch.randint(0, 256, (N, K // 2), dtype=torch.uint8, device=dev, generator=gen)
         ws = torch.randint(118, 126, (N, K // 32), dtype=torch.uint8, device=dev, generator=gen)
         w = mxfp4.prepare(mxfp4.MX4(wq, ws, N, K))
@@ -951,7 +951,7 @@ def main():
     ap.add_argument("--graph", action="store_true", help="time the pass as a replayed CUDA graph (decode rows)")
     ap.add_argument("--detail", action="store_true", help="per-shape GEMM table instead of the JSON line")
     ap.add_argument("--probe", default=None, help="one kernel case, a few eager launches (for ncu)")
-    ap.add_argument("--probe-rows", type=int, default=None, help="activation rows of the W4A8 decode probes")
+    ap.add_argument("--probe-rows", type=int, default=None, help="activation rows of the GEMM probes")
     ap.add_argument("--detail-rows", default=None)
     ap.add_argument("--detail-head", action="store_true", help="add the vocabulary head (head_q8) to --detail")
     ap.add_argument("--detail-shapes", default=None)

@@ -323,8 +323,8 @@ int launch_tile(const int8_t* a, const float* a_s, const int8_t* w, const float*
     return PB_OK;
 }
 
-// The CTA-pair kernel (clusters of two): 256 x 256 tiles.  Opt-in with PRISM_B200_PAIR=1: under the 1 kW power cap it
-// sustains the same rate as the single-CTA tile kernel and is a little slower in short bursts.
+// CTA pairs with the activation rows on the tensor-memory lanes, 256 x 256 tiles.  Opt-in with PRISM_B200_PAIR=1, for comparison runs: its
+// row tiles do not follow the rows there are, and it sustains the tile kernel's rate, not w8a8_tpair_kernel's.
 bool pair_enabled() {
     static int v = -1;
     if (v < 0) {
@@ -366,7 +366,7 @@ bool tpair_enabled() {
 
 // Cycles of w8a8_tpair_kernel with row tiles of nt: rounds of pairs, each as long as its stages or the drain of the tile before, and the
 // last drain.  Fitted to 26 projections at 65 to 4,096 rows: a stage's MMAs take 2.06 nt, its copies and barriers 355 + nt / 4; with
-// more rounds the copies of all pairs bound it at 256 + nt; a row of a tile drains in 42.
+// more rounds it is 256 + nt where that is more (all pairs' copies, the clock under the power cap); a row of a tile drains in 42.
 long tpair_cycles(int M, int N, int K, int nt) {
     const long KB = (K + 127) / 128, pairs = sm_count() / 2;
     const long rounds = ((long)((N + 255) / 256) * ((M + nt - 1) / nt) + pairs - 1) / pairs;

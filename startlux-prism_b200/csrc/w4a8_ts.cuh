@@ -47,6 +47,7 @@ struct TsCfg {
     // four expander and eight epilogue warps: 128 registers a thread.  With eight and sixteen the expanders wait for most of their time
     // and the accumulators are read no sooner (34816 x 5120 at 2,048 rows 944 -> 1,148 us).
     static constexpr int EXPW = 4, EPIW = 8, CG = EPIW / 4;              // CG: column groups of a unit
+    static_assert(16 % (8 * CG) == 0, "a warp's share of 16 rows is read eight columns at a time");
     static constexpr int EXP0 = 2, EPI0 = EXP0 + EXPW;
     static constexpr int THREADS = (EPI0 + EPIW) * 32;
     static constexpr int SETC = (Q4 ? 3 : 2) * NBU;                      // columns of an accumulator set: P0 | P1 (| mins)
@@ -478,7 +479,7 @@ w4a8_ts_kernel(const __grid_constant__ TsMaps maps, const TsArgs p) {
                     const uint32_t set = lane_base + e * C::SETC + ch * cw[h];
                     const float* av = s + 64 + h * C::AW;
 #pragma unroll
-                    for (int c = 0; c < C::AW; c += 8) {                 // past cw: the neighbour's columns, read and not stored
+                    for (int c = 0; c < C::AW; c += 8) {                 // cw is a multiple of 8: no column of a neighbour is read
                         if (c >= cw[h]) break;
                         uint32_t p0[8], p1[8], mf[8];
                         tmem_ld8(set + c, p0);

@@ -470,6 +470,33 @@ def test_many_rows_split_is_run(dev, M, N, K, split):
         assert bool((ws != 0x55).any()) and not bool(counters.any())
 
 
+@pytest.mark.parametrize("M,N,live", [(1024, 5120, 1000), (700, 9472, 700)])
+def test_tile_kernel_last_wave_split(dev, M, N, live):
+    """The tile kernel where the CTA pairs run by default (PRISM_B200_TPAIR=0 before the library's first GEMM): tiles 192 and 256 wide, the last
+    wave's tiles split along K in the device's workspace, bf16 stores and residual adds.  Run in a child process so the switch is read
+    afresh."""
+    import os
+    import subprocess
+    import sys
+    if os.environ.get("PRISM_B200_TPAIR") != "0":
+        env = dict(os.environ, PRISM_B200_TPAIR="0")
+        r = subprocess.run([sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", __file__, "-k",
+                            f"test_tile_kernel_last_wave_split and {M}-{N}-{live}"], env=env, capture_output=True, text=True)
+        assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-2000:]
+        return
+    K = 12304
+    a, w, sa, sw = (t.to(dev) for t in rand_w8a8(M, N, K, seed=M))
+    ref = ((a.double() @ w.double().T).float() * sa.view(-1, 1)) * sw.view(1, -1)
+    nr, (ws, counters) = n_rows(live, dev), w8a8._workspace(dev)
+    for epi in (0, 1):
+        base = torch.full((M, N), 0.5, dtype=(torch.bfloat16, torch.float32)[epi], device=dev)
+        out = base.clone()
+        ws.fill_(0x55)
+        w8a8.gemm(a, sa.view(-1), w, sw.view(-1), out, nr, K, epi=epi)
+        assert same(out[:live], base[:live] + ref[:live] if epi else ref[:live].bfloat16()) and same(out[live:], base[live:])
+        assert bool((ws != 0x55).any()) and not bool(counters.any())
+
+
 @pytest.mark.parametrize("M,N,K,off", [(100, 512, 17408, 0), (200, 640, 1040, 1), (1100, 5121, 272, 3), (333, 5120, 5120, 2)])
 def test_many_rows_add_keeps_subnormals(dev, M, N, K, off):
     """Residual adds into an output that the copy engine cannot address (odd offset or stride), or of one round of tiles that share a long K,
